@@ -257,10 +257,13 @@ struct mmdg_context {
   // buckets: per pair-class list, slots grouped by primitive count; per class
   // (bra group, ket group) buckets with their offsets inside the class region
   std::vector<int> ngroup;
+  std::vector<std::vector<int>> group_start, group_prims;  // per class list: first slot (one molecule) and largest
+                                                           // primitive count of every group
   DevBuf<int> d_gslot[kNumPairClasses];
   std::vector<int> kbase, nkeys;
   int total_keys = 0;
   DevBuf<long long> d_keyoff;
+  DevBuf<int> d_keyw;  // primitive quartets of a quartet of the bucket
   DevBuf<unsigned> d_qn;  // [2*total_keys]: FP64 and FP32 bucket lengths
   DevBuf<unsigned long long> d_work;  // [2*MMDG_NCLASS]: work counters of the FP64 and FP32 class launches
   Geometry geom() const {
@@ -454,10 +457,8 @@ __global__ void k_sqrt_screen(const double* screen, double* sq, float* sqf, long
 }
 
 // ------------------------------------------------------------------ set basis
-// At most kMaxGroups primitive-count groups per pair-class list, so that a class has
-// at most kMaxGroups^2 (bra group, ket group) buckets.
-static const int kMaxGroups = 16;
-
+// (at most kMaxGroups primitive-count groups per pair-class list, so that a class has
+// at most kMaxGroups^2 (bra group, ket group) buckets)
 // Partition of the sorted distinct primitive counts vals (with their frequencies)
 // into at most gmax contiguous ranges minimising the idle lane iterations
 // sum_t freq_t (max of its range - vals_t); returns the range index of every value.
@@ -493,6 +494,15 @@ static std::vector<int> group_counts(const std::vector<int>& vals, const std::ve
     j = i - 1;
   }
   return grp;
+}
+
+// lanes per pair (as a power of two) of the Schwarz kernel, whose heaviest pair has `most`
+// primitive pairs: a lane keeps about four of its most^2 primitive quartets.  One thread
+// per pair was a serial chain of up to 1296 of them, 1.35 ms of (H2O)8's set-up.
+static int schwarz_lanes(int most) {
+  int lg = 0;
+  while (lg < 5 && (long long)most * most > (4LL << lg)) ++lg;
+  return lg;
 }
 
 extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, int nshell, const int* shell_mol,
@@ -641,7 +651,9 @@ extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, i
       const ClassEntry* ce = nullptr;
       for (const ClassEntry& e : kClasses)
         if (pair_class(e.la, e.lb) == c && pair_class(e.lc, e.ld) == c) ce = &e;
-      CUDA_TRY(ce->schwarz(g, sa, tmp[c].p, (int)lists[c].size(), 0));
+      int most = 1;
+      for (int p : lists[c]) most = std::max(most, h->pr_count[p]);
+      CUDA_TRY(ce->schwarz(g, sa, tmp[c].p, (int)lists[c].size(), schwarz_lanes(most), 0));
     }
     CUDA_TRY(cudaDeviceSynchronize());
   }
@@ -698,7 +710,7 @@ extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, i
         const ClassEntry* ce = nullptr;
         for (const ClassEntry& e : kClasses)
           if (pair_class(e.la, e.lb) == c && pair_class(e.lc, e.ld) == c) ce = &e;
-        CUDA_TRY(ce->schwarz(gx, sx, dlist[c].p, (int)xl[c].size(), 0));
+        CUDA_TRY(ce->schwarz(gx, sx, dlist[c].p, (int)xl[c].size(), 0, 0));
       }
       CUDA_TRY(cudaDeviceSynchronize());
       CUDA_TRY(cudaMemcpy(qp.data(), dqp.p, sizeof(float) * npp, cudaMemcpyDeviceToHost));
@@ -767,6 +779,8 @@ extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, i
   CUDA_TRY(cudaMemcpy(Q.data(), h->d_Q.p, sizeof(float) * h->npair, cudaMemcpyDeviceToHost));
   h->cls_count.assign(kNumPairClasses, 0);
   h->ngroup.assign(kNumPairClasses, 0);
+  h->group_start.assign(kNumPairClasses, {});
+  h->group_prims.assign(kNumPairClasses, {});
   std::vector<std::vector<int>> slot_group(kNumPairClasses), slot_mol(kNumPairClasses);
   for (int c = 0; c < kNumPairClasses; ++c) {
     std::vector<int>& v = lists[c];
@@ -804,6 +818,12 @@ extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, i
       ms[i] = shell_mol[h->pa[v[i]]];
     }
     h->ngroup[c] = vals.empty() ? 0 : grp.back() + 1;
+    h->group_start[c].assign(h->ngroup[c] + 1, (int)v.size());
+    h->group_prims[c].assign(h->ngroup[c], 0);
+    for (size_t i = v.size(); i-- > 0;) {
+      h->group_start[c][gs[i]] = (int)i;
+      h->group_prims[c][gs[i]] = std::max(h->group_prims[c][gs[i]], h->pr_count[v[i]]);
+    }
     if (h->d_gslot[c].upload(gs) != cudaSuccess) return fail(MMDG_E_NOMEM, "mmdg_set_basis: allocation");
     slot_group[c] = gs;
     slot_mol[c] = ms;
@@ -862,7 +882,7 @@ extern "C" int mmdg_device_bytes(mmdg_context* h, long long* bytes) {
   MMDG_ADD(d_pa); MMDG_ADD(d_pb); MMDG_ADD(d_prb); MMDG_ADD(d_prc); MMDG_ADD(d_eoff);
   MMDG_ADD(d_pP); MMDG_ADD(d_pPf); MMDG_ADD(d_E64); MMDG_ADD(d_E32); MMDG_ADD(d_Q);
   MMDG_ADD(d_mol_shell0); MMDG_ADD(d_screen); MMDG_ADD(d_sq); MMDG_ADD(d_sqf); MMDG_ADD(d_dPf); MMDG_ADD(d_Dsh);
-  MMDG_ADD(d_counters); MMDG_ADD(d_q64); MMDG_ADD(d_q32); MMDG_ADD(d_keyoff); MMDG_ADD(d_qn); MMDG_ADD(d_work);
+  MMDG_ADD(d_counters); MMDG_ADD(d_q64); MMDG_ADD(d_q32); MMDG_ADD(d_keyoff); MMDG_ADD(d_keyw); MMDG_ADD(d_qn); MMDG_ADD(d_work);
   MMDG_ADD(d_pair_owner); MMDG_ADD(d_pair_canon);
   for (int c = 0; c < kNumPairClasses; ++c) {
     MMDG_ADD(d_cls[c]); MMDG_ADD(d_cls_moff[c]); MMDG_ADD(d_gslot[c]);
@@ -896,7 +916,14 @@ extern "C" int mmdg_eri_tensor(mmdg_context* h, double* out, void* stream) {
     const int cb = pair_class(e.la, e.lb), ck = pair_class(e.lc, e.ld);
     if (!h->cls_count[cb] || !h->cls_count[ck]) continue;
     ClassLaunch cl{h->d_cls[cb].p, h->d_cls[ck].p, h->cls_count[cb], h->cls_count[ck], cb == ck, 0.f, 0.f};
-    CUDA_TRY(e.tensor(g, t, cl, st));
+    TensorBuckets tb;
+    tb.nbg = h->ngroup[cb];
+    tb.nkg = h->ngroup[ck];
+    std::copy(h->group_start[cb].begin(), h->group_start[cb].end(), tb.bstart);
+    std::copy(h->group_start[ck].begin(), h->group_start[ck].end(), tb.kstart);
+    std::copy(h->group_prims[cb].begin(), h->group_prims[cb].end(), tb.bw);
+    std::copy(h->group_prims[ck].begin(), h->group_prims[ck].end(), tb.kw);
+    CUDA_TRY(e.tensor(g, t, cl, tb, st));
   }
   return MMDG_OK;
 }
@@ -1073,6 +1100,7 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
     h->kbase.assign(MMDG_NCLASS, 0);
     h->nkeys.assign(MMDG_NCLASS, 0);
     std::vector<long long> koff;
+    std::vector<int> kw;
     long long tot = 0;
     int nk = 0;
     for (int ci = 0; ci < MMDG_NCLASS; ++ci) {
@@ -1081,6 +1109,9 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
       h->q_off[ci] = tot;
       h->kbase[ci] = nk;
       h->nkeys[ci] = (int)cap.size();
+      const ClassEntry& e = kClasses[ci];
+      for (int wb : h->group_prims[pair_class(e.la, e.lb)])
+        for (int wk : h->group_prims[pair_class(e.lc, e.ld)]) kw.push_back(wb * wk);
       long long rel = 0;
       for (long long c2 : cap) {
         koff.push_back(rel);
@@ -1094,7 +1125,8 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
     h->total_keys = nk;
     if (h->d_q64.alloc(tot > 0 ? tot : 1) != cudaSuccess || h->d_qn.alloc(2 * (nk > 0 ? nk : 1)) != cudaSuccess ||
         h->d_work.alloc(2 * MMDG_NCLASS) != cudaSuccess ||
-        h->d_keyoff.upload(koff.empty() ? std::vector<long long>{0} : koff) != cudaSuccess) {
+        h->d_keyoff.upload(koff.empty() ? std::vector<long long>{0} : koff) != cudaSuccess ||
+        h->d_keyw.upload(kw.empty() ? std::vector<int>{1} : kw) != cudaSuccess) {
       h->q_off.clear();
       return fail(MMDG_E_NOMEM, "mmdg_fock: cannot allocate the quartet lists");
     }
@@ -1144,15 +1176,16 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
     if (h->cls_count[cb] && h->cls_count[ck]) {
       ClassLaunch cl{h->d_cls[cb].p, h->d_cls[ck].p, h->cls_count[cb], h->cls_count[ck], cb == ck, 0.f, split,
                      h->d_cls_moff[ck].p};
-      const long long* ko = h->d_keyoff.p + h->kbase[ci];
+      const int kb = h->kbase[ci];
+      BucketList bl{h->d_q64.p + h->q_off[ci], h->d_qn.p + kb, h->d_keyoff.p + kb, h->d_keyw.p + kb, h->nkeys[ci]};
       const int grid = h->class_grid[ci], blk = h->class_block[ci], item = h->class_item[ci];
       f.work = h->d_work.p + 2 * ci;
-      CUDA_TRY(e.fock(0, g, f, cl, h->d_q64.p + h->q_off[ci], h->d_qn.p + h->kbase[ci], ko, h->nkeys[ci], grid, blk,
-                      item, cs));
+      CUDA_TRY(e.fock(0, g, f, cl, bl, grid, blk, item, cs));
       if (split > 0.f) {
         f.work = h->d_work.p + 2 * ci + 1;
-        CUDA_TRY(e.fock(1, g, f, cl, h->d_q32.p + h->q_off[ci], h->d_qn.p + h->total_keys + h->kbase[ci], ko,
-                        h->nkeys[ci], grid, blk, item, cs));
+        bl.list = h->d_q32.p + h->q_off[ci];
+        bl.count = h->d_qn.p + h->total_keys + kb;
+        CUDA_TRY(e.fock(1, g, f, cl, bl, grid, blk, item, cs));
       }
     }
     if (class_ms) CUDA_TRY(cudaEventRecord(ev[2 * ci + 1], st));

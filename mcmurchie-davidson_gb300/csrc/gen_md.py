@@ -427,20 +427,20 @@ def generate_instances(outdir, ngroups=6):
     files = []
     decl = ["// Generated by gen_md.py -- do not edit.", "#pragma once", '#include "md_kernels.cuh"',
             '#include "md_warp.cuh"', "namespace mmdg {",
-            "typedef cudaError_t (*fock_fn)(int, const Geometry&, const FockArgs&, const ClassLaunch&, const int2*, const unsigned*, const long long*, int, int, int, int, cudaStream_t);",
-            "typedef cudaError_t (*tensor_fn)(const Geometry&, const TensorArgs&, const ClassLaunch&, cudaStream_t);",
-            "typedef cudaError_t (*schwarz_fn)(const Geometry&, const SchwarzArgs&, const int*, int, cudaStream_t);",
+            "typedef cudaError_t (*fock_fn)(int, const Geometry&, const FockArgs&, const ClassLaunch&, const BucketList&, int, int, int, cudaStream_t);",
+            "typedef cudaError_t (*tensor_fn)(const Geometry&, const TensorArgs&, const ClassLaunch&, const TensorBuckets&, cudaStream_t);",
+            "typedef cudaError_t (*schwarz_fn)(const Geometry&, const SchwarzArgs&, const int*, int, int, cudaStream_t);",
             "typedef cudaError_t (*quartets_fn)(int, const Geometry&, const QuartetArgs&, const QuartetItem*, int, cudaStream_t);",
             "struct ClassEntry { int la, lb, lc, ld; fock_fn fock; tensor_fn tensor; schwarz_fn schwarz; quartets_fn quartets; };"]
     for g in range(ngroups):
         decl.append(f"cudaError_t init_group{g}();")
     for c in cls:
         s = "".join(map(str, c))
-        decl.append(f"cudaError_t launch_fock_{s}(int, const Geometry&, const FockArgs&, const ClassLaunch&, const int2*, const unsigned*, const long long*, int, int, int, int, cudaStream_t);")
-        decl.append(f"cudaError_t launch_tensor_{s}(const Geometry&, const TensorArgs&, const ClassLaunch&, cudaStream_t);")
+        decl.append(f"cudaError_t launch_fock_{s}(int, const Geometry&, const FockArgs&, const ClassLaunch&, const BucketList&, int, int, int, cudaStream_t);")
+        decl.append(f"cudaError_t launch_tensor_{s}(const Geometry&, const TensorArgs&, const ClassLaunch&, const TensorBuckets&, cudaStream_t);")
         decl.append(f"cudaError_t launch_quartets_{s}(int, const Geometry&, const QuartetArgs&, const QuartetItem*, int, cudaStream_t);")
         if c[:2] == c[2:]:
-            decl.append(f"cudaError_t launch_schwarz_{s}(const Geometry&, const SchwarzArgs&, const int*, int, cudaStream_t);")
+            decl.append(f"cudaError_t launch_schwarz_{s}(const Geometry&, const SchwarzArgs&, const int*, int, int, cudaStream_t);")
     decl.append("static const ClassEntry kClasses[] = {")
     for c in cls:
         s = "".join(map(str, c))
@@ -457,26 +457,26 @@ def generate_instances(outdir, ngroups=6):
         for c in grp:
             s = "".join(map(str, c))
             md = f"MD_{s}"
-            t.append(f"cudaError_t launch_fock_{s}(int prec, const Geometry& g, const FockArgs& f, const ClassLaunch& cl, const int2* list, const unsigned* count, const long long* koff, int nkeys, int grid, int block, int item, cudaStream_t st) {{")
+            t.append(f"cudaError_t launch_fock_{s}(int prec, const Geometry& g, const FockArgs& f, const ClassLaunch& cl, const BucketList& bl, int grid, int block, int item, cudaStream_t st) {{")
             if is_warp_class(c):
                 mw = f"MDW_{s}"
                 t.append("  (void)block;")
                 for real, cond in (("float", "if (prec)"), ("double", "else")):
                     k = f"k_fock_warp<{mw}<{real}>, {real}>"
                     sm = f"WarpSmem<{mw}<{real}>, {real}>::bytes()"
-                    t.append(f"  {cond} {k}<<<persistent_blocks({k}, {sm}, grid), kThreads, {sm}, st>>>(g, f, cl, list, count, koff, nkeys, item);")
+                    t.append(f"  {cond} {k}<<<persistent_blocks({k}, {sm}, grid), kThreads, {sm}, st>>>(g, f, cl, bl, item);")
             else:
                 t.append("  (void)item;")
                 t.append(f"  if ({md}<double>::RSMEM || block <= 0) block = kThreads;  // shared-memory R tables are sized for kThreads")
                 for real, cond in (("float", "if (prec)"), ("double", "else")):
                     k = f"k_fock<{md}<{real}>, {real}>"
                     sm = f"smem_bytes<{md}<{real}>, {real}>()"
-                    t.append(f"  {cond} {k}<<<persistent_blocks({k}, {sm}, grid, block), block, {sm}, st>>>(g, f, cl, list, count, koff, nkeys);")
+                    t.append(f"  {cond} {k}<<<persistent_blocks({k}, {sm}, grid, block), block, {sm}, st>>>(g, f, cl, bl);")
             t.append(f"  return cudaGetLastError();")
             t.append("}")
-            t.append(f"cudaError_t launch_tensor_{s}(const Geometry& g, const TensorArgs& a, const ClassLaunch& cl, cudaStream_t st) {{")
-            t.append(f"  dim3 grid(cl.nbra, (cl.nket + kThreads - 1) / kThreads, {md}<double>::NCHUNK);")
-            t.append(f"  k_tensor<{md}<double>><<<grid, kThreads, smem_bytes<{md}<double>, double>(), st>>>(g, a, cl);")
+            t.append(f"cudaError_t launch_tensor_{s}(const Geometry& g, const TensorArgs& a, const ClassLaunch& cl, const TensorBuckets& tb, cudaStream_t st) {{")
+            sm = f"smem_bytes<{md}<double>, double>()"
+            t.append(f"  k_tensor<{md}<double>><<<persistent_blocks(k_tensor<{md}<double>>, {sm}), kThreads, {sm}, st>>>(g, a, cl, tb);")
             t.append(f"  return cudaGetLastError();")
             t.append("}")
             t.append(f"cudaError_t launch_quartets_{s}(int prec, const Geometry& g, const QuartetArgs& a, const QuartetItem* items, int n, cudaStream_t st) {{")
@@ -496,8 +496,8 @@ def generate_instances(outdir, ngroups=6):
                 inits.append(f"  if ((e = cudaFuncSetAttribute(k_fock<{md}<float>, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<{md}<float>, float>()))) return e;")
             inits.append(f"  if ((e = cudaFuncSetAttribute(k_tensor<{md}<double>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<{md}<double>, double>()))) return e;")
             if c[:2] == c[2:]:
-                t.append(f"cudaError_t launch_schwarz_{s}(const Geometry& g, const SchwarzArgs& a, const int* list, int n, cudaStream_t st) {{")
-                t.append(f"  k_schwarz<{md}<double>><<<(unsigned)(((long long)n * {md}<double>::NCHUNK + kThreads - 1) / kThreads), kThreads, smem_bytes<{md}<double>, double>(), st>>>(g, a, list, n);")
+                t.append(f"cudaError_t launch_schwarz_{s}(const Geometry& g, const SchwarzArgs& a, const int* list, int n, int lg, cudaStream_t st) {{")
+                t.append(f"  k_schwarz<{md}<double>><<<(unsigned)(((((long long)n * {md}<double>::NCHUNK) << lg) + kThreads - 1) / kThreads), kThreads, smem_bytes<{md}<double>, double>(), st>>>(g, a, list, n, lg);")
                 t.append(f"  return cudaGetLastError();")
                 t.append("}")
                 inits.append(f"  if ((e = cudaFuncSetAttribute(k_schwarz<{md}<double>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<{md}<double>, double>()))) return e;")

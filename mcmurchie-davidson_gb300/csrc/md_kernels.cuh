@@ -4,13 +4,14 @@
 // walks every candidate (bra shell pair, ket shell pair) of the class and appends
 // the survivors of the Schwarz x density bound to bucketed quartet lists (buckets
 // keyed by the primitive-count groups of the two pairs, FP64 and FP32 lists); then
-// k_fock, a persistent kernel, evaluates the list, one thread per (quartet, ket
-// chunk), chunk-major, so a warp shares its code path and, inside a bucket, its
-// primitive trip counts.  Short lists and FP32 lists are split by grid stride; long
-// FP64 lists are handed out 32 quartets per warp from an atomic counter, so the SMs
-// finish together.  The classes above L = 4 have a warp-cooperative Fock kernel of
-// their own (md_warp.cuh).  The ERI tensor, the Schwarz table and listed quartets
-// use one thread per shell quartet.
+// k_fock, a persistent kernel, evaluates the list, 1 to 32 lanes per (quartet, ket
+// chunk) (the lanes share the quartet's primitive pairs, see plan_buckets),
+// chunk-major, so a warp shares its code path and, inside a bucket, its primitive
+// trip counts.  FP32 lists are split by grid stride; FP64 lists are claimed 32 lanes per
+// warp from an atomic counter, so the SMs finish together.  The classes above L = 4 have
+// a warp-cooperative Fock kernel of their own (md_warp.cuh).  The ERI tensor enumerates the same buckets without a list (nothing
+// is screened), the Schwarz table runs a warp-wide group per heavy pair; listed
+// quartets use one thread per shell quartet.
 #pragma once
 #include "md_device.cuh"
 #include "md_gen.cuh"
@@ -128,90 +129,190 @@ static __global__ void __launch_bounds__(kThreads) k_screen(Geometry g, FockArgs
 }
 
 constexpr int kMaxKeys = 256;
+constexpr int kMaxGroups = 16;  // primitive-count groups per pair-class list (kMaxGroups^2 <= kMaxKeys)
 
-// Evaluation of a bucketed quartet list: persistent loop over (chunk, bucket,
-// quartet), chunk-major, so that a warp shares its chunk (code path) and, inside a
-// bucket, its primitive trip counts; heaviest buckets first.
-//
-// FP64 lists of at least 8 items per thread claim their work dynamically: each warp
-// takes the next 32 items from the launch's counter (one atomic per claim, issued one
-// claim ahead so its round trip overlaps the work), lane l the item base + l.  With
-// the static grid-stride split the average SM sat idle for 20 % of a (ps|ss) launch
-// while the slowest finished (ncu: sm__cycles_active avg 9.9M, max 12.4M cycles of
-// 12.4M); with the warp kernel's claims (md_warp.cuh) it cut the (H2O)16 class kernels
-// run one after another from 44.9 to 38.6 ms and the 4-stream build from 36.4 to
-// 34.9 ms (same GPU, two repeats each).  Claims of 128 or 256 items were 1.8-2.7x
-// slower (the warps' working set of pairs and E' rows spreads over that many more
-// quartets); short lists (a few items per thread: the near quartets of a mixed
-// build) and the memory-latency-bound FP32 lists ran 5-35 % slower with claims, so
-// they keep the static split.
-template <class MD, typename Real>
-__global__ void __launch_bounds__(kMaxFockBlock) k_fock(Geometry g, FockArgs f, ClassLaunch cl, const int2* list,
-                                                   const unsigned* count, const long long* key_off, int nkeys) {
-  __shared__ unsigned s_pre[kMaxKeys + 1];
-  __shared__ long long s_off[kMaxKeys];
-  if (threadIdx.x == 0) {
+// One bucketed list of a class: bucket k holds count[k] quartets from key_off[k] on, each
+// of about key_w[k] primitive quartets.
+struct BucketList {
+  const int2* list;
+  const unsigned* count;
+  const long long* key_off;
+  const int* key_w;
+  int nkeys;
+};
+
+// How a launch walks its buckets: position x (heaviest bucket, stored last, first) covers
+// the work items pre[x] .. pre[x + 1), a multiple of 32, of bucket nkeys - 1 - x, with
+// 2^lg[x] lanes per quartet.
+struct BucketPlan {
+  unsigned pre[kMaxKeys + 1];
+  unsigned char lg[kMaxKeys];
+};
+
+// Lanes per quartet.  A quartet of w primitive quartets on one thread is a serial chain of
+// w x ~1.1 us, whatever the rest of the GPU does: an oxygen-core (ss|ss) quartet (1296)
+// took 1.4 ms, which alone was the length of that class's launch on (H2O)4 and of most
+// classes on one molecule.  So a bucket's quartets get the smallest power of two of lanes
+// (up to 32) that brings a lane below twice the launch's average work per thread (never
+// below kLanePrims primitive quartets: a shorter share costs more in digestion and sums
+// over the lanes than it saves).  Long lists thus keep one lane per quartet except for
+// the few heavy buckets that would run on after the others.  Measured (ms per build, 8
+// streams; share of 1/4, 1/2, 1, 2 averages, sums over the lanes): (H2O)4 6-31G** 1.87,
+// 1.52, 1.44, 1.30; (H2O)16 with FP32 below 1e-5 24.4, 23.3, 22.6, 22.3; kLanePrims 2, 4,
+// 8 on (H2O)4: 2.45, 1.44, 1.33, 4 the better on one stream.  One thread per quartet: 2.74.
+constexpr float kLanePrims = 4.0f;
+
+template <class CountF, class WeightF>
+__device__ __forceinline__ void plan_buckets(BucketPlan& p, int nkeys, int nchunk, long long nthreads, CountF count,
+                                             WeightF weight) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    float W = 0.f;
+    for (int x = lane; x < nkeys; x += 32) W += float(count(nkeys - 1 - x)) * float(weight(nkeys - 1 - x));
+    for (int o = 16; o > 0; o >>= 1) W += __shfl_xor_sync(0xffffffffu, W, o);
+    const float share = fmaxf(kLanePrims, 2.0f * W * float(nchunk) / float(nthreads));
     unsigned acc = 0;
-    for (int k = 0; k < nkeys; ++k) {
-      s_pre[k] = acc;
-      s_off[k] = key_off[k];
-      acc += count[k];
+    for (int x0 = 0; x0 < nkeys; x0 += 32) {
+      const int x = x0 + lane;
+      unsigned len = 0;
+      int lg = 0;
+      if (x < nkeys) {
+        const unsigned c = count(nkeys - 1 - x);
+        const float w = float(weight(nkeys - 1 - x));
+        while (lg < 5 && w > share * float(1 << lg)) ++lg;
+        len = ((c << lg) + 31u) & ~31u;
+      }
+      unsigned end = len;
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, end, d);
+        if (lane >= d) end += t;
+      }
+      if (x < nkeys) {
+        p.pre[x] = acc + end - len;
+        p.lg[x] = (unsigned char)lg;
+      }
+      acc += __shfl_sync(0xffffffffu, end, 31);
     }
-    s_pre[nkeys] = acc;
+    if (lane == 0) p.pre[nkeys] = acc;
   }
   __syncthreads();
-  const unsigned n = s_pre[nkeys];
+}
+
+// The share of lane `sub` of a 2^lg-lane group: the bra primitive pairs are split first
+// (their transform runs once per bra pair), the ket ones among the remaining lanes.
+template <class C>
+__device__ __forceinline__ void split_primitives(C& c, int lg, int sub) {
+  if (lg == 0) return;
+  const int nb = c.bra_end - c.bra_begin, nk = c.ket_end - c.ket_begin;
+  const int lb = min(lg, 31 - __clz(nb)), lk = lg - lb;
+  const int sb = sub & ((1 << lb) - 1), sk = sub >> lb;
+  const int b0 = (sb * nb) >> lb, b1 = ((sb + 1) * nb) >> lb;
+  const int k0 = (sk * nk) >> lk, k1 = ((sk + 1) * nk) >> lk;
+  c.bra_end = c.bra_begin + (k1 > k0 ? b1 : b0);  // no ket pair left for this lane: nothing to do
+  c.bra_begin += b0;
+  c.ebra += (long long)b0 * c.nnz_ab;
+  c.ket_end = c.ket_begin + k1;
+  c.ket_begin += k0;
+  c.eket += (long long)k0 * c.nnz_cd;
+}
+
+// A digest behind a group of 2^lg lanes: every value is summed over the group, and the
+// lanes take turns in digesting the sums.
+template <class Digest>
+struct GroupDigest {
+  Digest& d;
+  int lanes, sub;
+  unsigned mask;
+  int turn;
+  __device__ __forceinline__ GroupDigest(Digest& d_, int lg, int lane)
+      : d(d_), lanes(1 << lg), sub(lane & ((1 << lg) - 1)),
+        mask((lg == 5 ? 0xffffffffu : ((1u << (1 << lg)) - 1u)) << (lane & ~((1 << lg) - 1))), turn(0) {}
+  template <typename Real>
+  __device__ __forceinline__ void put(int ca, int cb, int cc, int cd, Real v) {
+    for (int o = 1; o < lanes; o <<= 1) v += __shfl_xor_sync(mask, v, o);
+    if ((turn++ & (lanes - 1)) == sub) d.put(ca, cb, cc, cd, v);
+  }
+};
+
+// Evaluation of a bucketed quartet list: persistent loop over (chunk, bucket, quartet),
+// chunk-major, so that a warp shares its chunk (code path) and its primitive trip
+// counts; heaviest buckets first.  The lanes of an FP64 quartet sum their integrals with
+// shuffles and take turns in digesting the sums (digesting every lane's partial integrals
+// instead, G being linear in them, rounds once per lane: the error of G against 64 bits
+// went from 5.6e-15 to 8.0e-15 on (H2O)4).  The one-lane path stays separate: the group's
+// bookkeeping in every digestion cost it 3-7 % on (H2O)16.  The lanes of an FP32 quartet
+// do digest partial integrals, which spares that kernel up to 40 registers.
+//
+// FP64 lists claim their work: each warp takes the next 32 items from the launch's
+// counter.  With a static grid-stride split the average SM sat idle for 20 % of a
+// (ps|ss) launch while the slowest finished (ncu: sm__cycles_active avg 9.9M, max 12.4M
+// cycles of 12.4M), and on several streams a block that starts late holds its share
+// back.  (Claiming one item ahead hid nothing more on long lists, and on short ones
+// left warps idle beside claimed work: mixed (H2O)16 26.7 -> 25.4 ms without.)  Claims of 128 or 256 items were 1.8-2.7x slower (the warps'
+// working set of pairs and E' rows spreads over that many more quartets).  The
+// memory-latency-bound FP32 lists keep the static split, neighbouring warps on
+// neighbouring quartets.
+template <class MD, typename Real>
+__global__ void __launch_bounds__(kMaxFockBlock) k_fock(Geometry g, FockArgs f, ClassLaunch cl, BucketList bl) {
+  __shared__ BucketPlan plan;
+  // block size: kThreads for classes with shared-memory R tables, else 64..256 (tile),
+  // a multiple of 32 either way, so every warp is full
+  const long long nthreads = (long long)gridDim.x * blockDim.x;
+  plan_buckets(plan, bl.nkeys, MD::NCHUNK, nthreads, [&](int k) { return __ldg(bl.count + k); },
+               [&](int k) { return __ldg(bl.key_w + k); });
+  __shared__ unsigned s_count[kMaxKeys];
+  __shared__ long long s_off[kMaxKeys];
+  for (int x = threadIdx.x; x < bl.nkeys; x += blockDim.x) {  // by plan position
+    s_count[x] = __ldg(bl.count + bl.nkeys - 1 - x);
+    s_off[x] = __ldg(bl.key_off + bl.nkeys - 1 - x);
+  }
+  __syncthreads();
+  const unsigned n = plan.pre[bl.nkeys];
   const long long total = (long long)n * MD::NCHUNK;
   extern __shared__ double smem_d[];
   Real* rs = reinterpret_cast<Real*>(smem_d) + threadIdx.x;
   unsigned nfq = 0, nsq = 0, npq = 0, nbp = 0, nas = 0;
-  int key = 0;
-  // block size: kThreads for classes with shared-memory R tables, else 64..256 (tile),
-  // a multiple of 32 either way, so every warp is full
-  const long long nthreads = (long long)gridDim.x * blockDim.x;
-  const bool dynamic = sizeof(Real) == 8 && total >= 8 * nthreads;
+  int x = 0;
+  constexpr bool kClaim = sizeof(Real) == 8;
   const unsigned lane = threadIdx.x & 31u;
-  unsigned long long base = 0, next = 0;
-  long long sidx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (dynamic) {
-    if (lane == 0) base = atomicAdd(f.work, 32ull);
-    base = __shfl_sync(0xffffffffu, base, 0);
-  }
-  for (;;) {
-    long long idx;
-    if (dynamic) {
-      if (base >= (unsigned long long)total) break;  // warp-uniform
-      if (lane == 0) next = atomicAdd(f.work, 32ull);  // the next claim, in flight during this one
-      idx = (long long)base + lane;
-    } else {
-      if (sidx >= total) break;
-      idx = sidx;
+  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;; idx += nthreads) {
+    if (kClaim) {
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(f.work, 32ull);
+      idx = (long long)__shfl_sync(0xffffffffu, base, 0) + lane;
     }
-    if (idx < total) {
-      const int chunk = (int)(idx / n);
-      // buckets run from the heaviest (most primitive pairs, stored last) to the
-      // lightest, so the loop's last rounds hold the cheapest quartets
-      const unsigned r = n - 1u - (unsigned)(idx - (long long)chunk * n);
-      if (r < s_pre[key]) key = 0;
-      while (r >= s_pre[key + 1]) ++key;
-      const int2 e = list[s_off[key] + (r - s_pre[key])];
+    if (idx >= total) break;  // warp-uniform: total is a multiple of 32
+    const int chunk = (int)(idx / n);
+    const unsigned r = (unsigned)(idx - (long long)chunk * n);
+    if (r < plan.pre[x]) x = 0;
+    while (r >= plan.pre[x + 1]) ++x;
+    const int lg = plan.lg[x];
+    const unsigned slot = (r - plan.pre[x]) >> lg;
+    if (slot < s_count[x]) {
+      const int2 e = bl.list[s_off[x] + (s_count[x] - 1u - slot)];
       const int bp = __ldg(cl.bra + e.x), kp = __ldg(cl.ket + e.y);
       const int sa = __ldg(g.pa + bp), sb = __ldg(g.pb + bp), sc = __ldg(g.pa + kp), sd = __ldg(g.pb + kp);
       Ctx<Real> c = make_ctx<MD, Real>(g, bp, kp, rs);
       c.chunk = MD::NCHUNK > 1 ? chunk : -1;
       QuartetInfo q{sa, sb, sc, sd, sa == sb, sc == sd, bp == kp, __ldg(g.sh_mol + sa)};
       FockDigest<ncart(MD::LB), ncart(MD::LD)> dg(g, f, q);
-      MD::run(c, dg);
-      nfq += dg.nfq;
+      const int sub = (int)lane & ((1 << lg) - 1);
+      split_primitives(c, lg, sub);
+      if (kClaim && lg > 0) {  // warp-uniform: a bucket fills whole warps
+        GroupDigest<FockDigest<ncart(MD::LB), ncart(MD::LD)>> gd(dg, lg, (int)lane);
+        MD::run(c, gd);
+        nfq += dg.nfq;
+      } else {
+        MD::run(c, dg);
+        if (sub == 0) nfq += dg.nfq;
+      }
       if (chunk == 0) {
-        ++nsq;
+        if (sub == 0) ++nsq;
         npq += unsigned((c.bra_end - c.bra_begin) * (c.ket_end - c.ket_begin));
         nbp += unsigned(c.bra_end - c.bra_begin);
         nas += c.nasym;
       }
     }
-    if (dynamic) base = __shfl_sync(0xffffffffu, next, 0);
-    else sidx += nthreads;
   }
   if (f.counters) {
     const unsigned mask = __activemask();
@@ -228,23 +329,67 @@ __global__ void __launch_bounds__(kMaxFockBlock) k_fock(Geometry g, FockArgs f, 
   }
 }
 
+// The buckets of an unscreened class of one molecule: its class lists are sorted by
+// primitive count, so group g of the bra list is the slots bstart[g] .. bstart[g + 1),
+// each of at most bw[g] primitive pairs; bucket k = gb * nkg + gk is the rectangle of two
+// groups (the triangle for a group with itself, nothing for gk > gb, when the lists are
+// the same).
+struct TensorBuckets {
+  int nbg, nkg;
+  int bstart[kMaxGroups + 1], kstart[kMaxGroups + 1];
+  int bw[kMaxGroups], kw[kMaxGroups];
+};
+
+// Every ERI of the class into the tensor, 1 to 32 lanes per (quartet, ket chunk) as in
+// k_fock, persistent over the buckets.  (One thread per quartet: N = 75 10.6 ms, its 21
+// launches each as long as their heaviest quartet; with groups 2.2 ms.)
 template <class MD>
-__global__ void __launch_bounds__(kThreads) k_tensor(Geometry g, TensorArgs t, ClassLaunch cl) {
-  const int ib = blockIdx.x;
-  const int jk = blockIdx.y * kThreads + threadIdx.x;
-  if (ib >= cl.nbra || jk >= cl.nket) return;
-  if (cl.same && jk > ib) return;
-  const int bp = __ldg(cl.bra + ib), kp = __ldg(cl.ket + jk);
-  const int sa = __ldg(g.pa + bp), sb = __ldg(g.pb + bp), sc = __ldg(g.pa + kp), sd = __ldg(g.pb + kp);
-  const int mol = __ldg(g.sh_mol + sa);
-  if (__ldg(g.sh_mol + sc) != mol) return;
+__global__ void __launch_bounds__(kThreads) k_tensor(Geometry g, TensorArgs t, ClassLaunch cl, TensorBuckets tb) {
+  __shared__ BucketPlan plan;
+  const int nkeys = tb.nbg * tb.nkg;
+  auto count = [&](int k) -> unsigned {
+    const int gb = k / tb.nkg, gk = k - gb * tb.nkg;
+    const unsigned a = tb.bstart[gb + 1] - tb.bstart[gb], b = tb.kstart[gk + 1] - tb.kstart[gk];
+    return !cl.same || gk < gb ? a * b : (gk == gb ? a * (a + 1) / 2 : 0u);
+  };
+  plan_buckets(plan, nkeys, MD::NCHUNK, (long long)gridDim.x * kThreads, count,
+               [&](int k) { return tb.bw[k / tb.nkg] * tb.kw[k % tb.nkg]; });
+  const unsigned n = plan.pre[nkeys];
+  const long long total = (long long)n * MD::NCHUNK, stride = (long long)gridDim.x * kThreads;
+  const unsigned lane = threadIdx.x & 31u;
   extern __shared__ double smem_d[];
   double* rs = smem_d + threadIdx.x;
-  Ctx<double> c = make_ctx<MD, double>(g, bp, kp, rs);
-  c.chunk = MD::NCHUNK > 1 ? (int)blockIdx.z : -1;  // one ket chunk per grid z-slice
-  QuartetInfo q{sa, sb, sc, sd, sa == sb, sc == sd, bp == kp, mol};
-  TensorDigest<ncart(MD::LB), ncart(MD::LD)> dg(g, t, q);
-  MD::run(c, dg);
+  int x = 0;
+  for (long long idx = ((long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + lane; idx < total; idx += stride) {
+    const int chunk = (int)(idx / n);
+    const unsigned r = (unsigned)(idx - (long long)chunk * n);
+    if (r < plan.pre[x]) x = 0;
+    while (r >= plan.pre[x + 1]) ++x;
+    const int lg = plan.lg[x], key = nkeys - 1 - x;
+    const unsigned slot = (r - plan.pre[x]) >> lg;
+    if (slot >= count(key)) continue;
+    const int gb = key / tb.nkg, gk = key - gb * tb.nkg;
+    int ib, jk;
+    if (cl.same && gb == gk) {  // slot = ib (ib + 1) / 2 + jk
+      ib = (int)((sqrtf(8.0f * float(slot) + 1.0f) - 1.0f) * 0.5f);
+      while ((long long)ib * (ib + 1) / 2 > (long long)slot) --ib;
+      while ((long long)(ib + 1) * (ib + 2) / 2 <= (long long)slot) ++ib;
+      jk = (int)((long long)slot - (long long)ib * (ib + 1) / 2);
+    } else {
+      const unsigned b = tb.kstart[gk + 1] - tb.kstart[gk];
+      ib = (int)(slot / b);
+      jk = (int)(slot - (unsigned)ib * b);
+    }
+    const int bp = __ldg(cl.bra + tb.bstart[gb] + ib), kp = __ldg(cl.ket + tb.kstart[gk] + jk);
+    const int sa = __ldg(g.pa + bp), sb = __ldg(g.pb + bp), sc = __ldg(g.pa + kp), sd = __ldg(g.pb + kp);
+    Ctx<double> c = make_ctx<MD, double>(g, bp, kp, rs);
+    c.chunk = MD::NCHUNK > 1 ? chunk : -1;
+    QuartetInfo q{sa, sb, sc, sd, sa == sb, sc == sd, bp == kp, __ldg(g.sh_mol + sa)};
+    TensorDigest<ncart(MD::LB), ncart(MD::LD)> dg(g, t, q);
+    GroupDigest<TensorDigest<ncart(MD::LB), ncart(MD::LD)>> gd(dg, lg, (int)lane);
+    split_primitives(c, lg, gd.sub);
+    MD::run(c, gd);
+  }
 }
 
 // listed shell quartets of one class (mmdg_eri_quartets): one thread per (item, ket
@@ -263,11 +408,11 @@ __global__ void __launch_bounds__(kThreads) k_quartets(Geometry g, QuartetArgs a
   MD::run(c, dg);
 }
 
-// diagonal quartets (ab|ab) of one pair class: the Schwarz table
-// (one thread per (pair, ket chunk), chunk-major)
+// diagonal quartets (ab|ab) of one pair class: the Schwarz table.  2^lg lanes per (pair,
+// ket chunk), chunk-major; whole groups leave together
 template <class MD>
-__global__ void __launch_bounds__(kThreads) k_schwarz(Geometry g, SchwarzArgs s, const int* list, int n) {
-  const long long idx = blockIdx.x * (long long)kThreads + threadIdx.x;
+__global__ void __launch_bounds__(kThreads) k_schwarz(Geometry g, SchwarzArgs s, const int* list, int n, int lg) {
+  const long long idx = (blockIdx.x * (long long)kThreads + threadIdx.x) >> lg;
   if (idx >= (long long)n * MD::NCHUNK) return;
   const int chunk = (int)(idx / n);
   const int bp = __ldg(list + (idx - (long long)chunk * n));
@@ -278,7 +423,9 @@ __global__ void __launch_bounds__(kThreads) k_schwarz(Geometry g, SchwarzArgs s,
   c.chunk = MD::NCHUNK > 1 ? chunk : -1;
   QuartetInfo q{sa, sb, sa, sb, sa == sb, sa == sb, true, __ldg(g.sh_mol + sa)};
   SchwarzDigest<ncart(MD::LB), ncart(MD::LD)> dg(g, s, q, bp);
-  MD::run(c, dg);
+  GroupDigest<SchwarzDigest<ncart(MD::LB), ncart(MD::LD)>> gd(dg, lg, (int)(threadIdx.x & 31));
+  split_primitives(c, lg, gd.sub);
+  MD::run(c, gd);
 }
 
 template <class MD, typename Real>

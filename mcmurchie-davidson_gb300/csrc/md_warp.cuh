@@ -58,9 +58,8 @@ struct WarpSmem {
 };
 
 template <class MD, typename Real>
-__global__ void __launch_bounds__(kThreads) k_fock_warp(Geometry g, FockArgs f, ClassLaunch cl, const int2* list,
-                                                        const unsigned* count, const long long* key_off,
-                                                        int nkeys, int max_item) {
+__global__ void __launch_bounds__(kThreads) k_fock_warp(Geometry g, FockArgs f, ClassLaunch cl, BucketList bl,
+                                                        int max_item) {
   constexpr int L = MD::L, HL = MD::HL, HP = MD::HP, NAB = MD::NAB, NCD = MD::NCD;
   constexpr int NB = ncart(MD::LB), ND = ncart(MD::LD);
   constexpr int NKO = (NCD * HP + 31) / 32;  // ket-transform passes
@@ -70,14 +69,24 @@ __global__ void __launch_bounds__(kThreads) k_fock_warp(Geometry g, FockArgs f, 
   __shared__ long long s_off[kMaxKeys];
   __shared__ unsigned s_ket[NCD], s_bra[NAB];
   __shared__ short s_herm[HL];  // packed (t | u << 5 | v << 10) of every Hermite index
-  if (threadIdx.x == 0) {
+  const int nkeys = bl.nkeys;
+  if (threadIdx.x < 32) {  // exclusive prefix sum of the bucket lengths
     unsigned acc = 0;
-    for (int k = 0; k < nkeys; ++k) {
-      s_pre[k] = acc;
-      s_off[k] = key_off[k];
-      acc += count[k];
+    for (int k0 = 0; k0 < nkeys; k0 += 32) {
+      const int k = k0 + threadIdx.x;
+      const unsigned len = k < nkeys ? bl.count[k] : 0u;
+      unsigned end = len;
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, end, d);
+        if ((int)threadIdx.x >= d) end += t;
+      }
+      if (k < nkeys) {
+        s_pre[k] = acc + end - len;
+        s_off[k] = bl.key_off[k];
+      }
+      acc += __shfl_sync(0xffffffffu, end, 31);
     }
-    s_pre[nkeys] = acc;
+    if (threadIdx.x == 0) s_pre[nkeys] = acc;
   }
   for (int x = threadIdx.x; x < NCD; x += kThreads) s_ket[x] = MD::ket_pair(x);
   for (int x = threadIdx.x; x < NAB; x += kThreads) s_bra[x] = MD::bra_pair(x);
@@ -118,7 +127,7 @@ __global__ void __launch_bounds__(kThreads) k_fock_warp(Geometry g, FockArgs f, 
       const unsigned qi = n - 1u - (q0 + lane);  // heaviest buckets (stored last) first
       int key = 0;
       while (qi >= s_pre[key + 1]) ++key;
-      const int2 e = list[s_off[key] + (qi - s_pre[key])];
+      const int2 e = bl.list[s_off[key] + (qi - s_pre[key])];
       qbp = __ldg(cl.bra + e.x);
       qkp = __ldg(cl.ket + e.y);
       qnp = __ldg(g.pr_count + qbp) * __ldg(g.pr_count + qkp);

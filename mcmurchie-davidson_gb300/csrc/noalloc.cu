@@ -98,6 +98,19 @@ int nnz_pair_na(int la, int lb) {
   return n;
 }
 
+// Groups of equal primitive count of a sorted class list (the last one takes the rest):
+// first slot and largest count of each; returns how many.
+int na_groups(const int* prc, const int* list, int n, int* start, int* prims) {
+  int g = -1;
+  for (int x = 0; x < n; ++x) {
+    const int k = prc[list[x]];
+    if (g < 0 || (k != prims[g] && g + 1 < kMaxGroups)) start[++g] = x;
+    prims[g] = k;
+  }
+  start[g + 1] = n;
+  return g + 1;
+}
+
 }  // namespace
 
 static_assert(kNoAllocScratchBytes == 1738240, "scratch size stated in include/mmdg.h");
@@ -184,7 +197,11 @@ extern "C" int mmdg_eri_tensor_noalloc(int nshell, const int* shell_L, const int
     for (int c = 0; c < kNA_PairClasses; ++c) {
       lbeg[c] = n;
       for (int p = 0; p < npair; ++p)
-        if (pcls[p] == c) lists[n++] = p;
+        if (pcls[p] == c) {  // by primitive count, as k_tensor's buckets want them
+          int x = n++;
+          for (; x > lbeg[c] && prc[lists[x - 1]] > prc[p]; --x) lists[x] = lists[x - 1];
+          lists[x] = p;
+        }
     }
     lbeg[kNA_PairClasses] = n;
   }
@@ -336,7 +353,10 @@ extern "C" int mmdg_eri_tensor_noalloc(int nshell, const int* shell_L, const int
     const int nb = lbeg[cb + 1] - lbeg[cb], nk = lbeg[ck + 1] - lbeg[ck];
     if (!nb || !nk) continue;
     ClassLaunch cl{dlist + lbeg[cb], dlist + lbeg[ck], nb, nk, cb == ck, 0.f, 0.f};
-    NA_TRY(ce.tensor(g, t, cl, st));
+    TensorBuckets tb;
+    tb.nbg = na_groups(prc, lists + lbeg[cb], nb, tb.bstart, tb.bw);
+    tb.nkg = na_groups(prc, lists + lbeg[ck], nk, tb.kstart, tb.kw);
+    NA_TRY(ce.tensor(g, t, cl, tb, st));
   }
 #undef NA_TRY
   return MMDG_OK;

@@ -16,7 +16,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "_lib", "libmmdg.so")
 NCLASS = 21
 NCOUNT = 5  # per-class counters of a Fock build (mmdg_fock)
-DEFAULT_STREAMS_SINGLE = 4
+DEFAULT_STREAMS_SINGLE = 8
 MAX_COMP = 6
 LMAX = 2
 
@@ -132,9 +132,10 @@ class Context:
             check(lib().mmdg_set_basis(h, self.nmol, _ptr(self.nfunc), self.nshell, _ptr(mol), _ptr(L), _ptr(K),
                                        _ptr(cen), _ptr(ex), _ptr(co), _ptr(fn)), "mmdg_set_basis")
         if self.nmol == 1:
-            # one molecule: the class kernels of a Fock build run on four concurrent
-            # streams (the autotuner's choice on (H2O)16 / 6-31G**: 52.7 against 62.1 ms
-            # per build in FP64, 31.4 against 43.5 ms mixed); batched contexts keep one
+            # one molecule: the class kernels of a Fock build run on eight concurrent
+            # streams ((H2O)4 / 6-31G** 3.3, 2.0, 1.55, 1.30 ms per build on 1, 2, 4, 8;
+            # (H2O)16 46.7, 45.0, 44.9, 45.0 in FP64); batched contexts keep one, their
+            # launches fill the GPU
             check(lib().mmdg_set_streams(h, DEFAULT_STREAMS_SINGLE), "mmdg_set_streams")
         self.nn = int(np.sum(self.nfunc.astype(np.int64) ** 2))
         self.ntri = int(np.sum(self.nfunc.astype(np.int64) * (self.nfunc + 1) // 2))
