@@ -215,6 +215,10 @@ struct mmdg_context {
   std::vector<long long> e_off;
   std::vector<int> pair_row;  // pair index of (s1, s1); (s1, s2 <= s1) is pair_row[s1] + s1 - s2
   std::vector<int> shell_L, shell_molv;
+  std::vector<int> shell_K, shell_poff;             // host copies for the gradient's primitive pairs
+  std::vector<double> shell_center, prim_exp;
+  std::mutex grad_mu;                               // one gradient of a context at a time:
+  DevBuf<unsigned char> d_grad;                     // its workspace
   DevBuf<int> d_pa, d_pb, d_prb, d_prc;
   DevBuf<long long> d_eoff;
   DevBuf<double4_32a> d_pP;
@@ -571,6 +575,10 @@ extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, i
   h->pair_row.assign(nshell, 0);
   h->shell_L.assign(shell_L, shell_L + nshell);
   h->shell_molv.assign(shell_mol, shell_mol + nshell);
+  h->shell_K.assign(shell_nprim, shell_nprim + nshell);
+  h->shell_poff = poff;
+  h->shell_center.assign(shell_center, shell_center + 3 * (size_t)nshell);
+  h->prim_exp.assign(prim_exp, prim_exp + total_prim);
   for (int s1 = 0; s1 < nshell; ++s1) {
     h->pair_row[s1] = (int)h->pa.size();
     for (int s2 = s1; s2 >= 0 && shell_mol[s2] == shell_mol[s1]; --s2) {
@@ -883,7 +891,7 @@ extern "C" int mmdg_device_bytes(mmdg_context* h, long long* bytes) {
   MMDG_ADD(d_pP); MMDG_ADD(d_pPf); MMDG_ADD(d_E64); MMDG_ADD(d_E32); MMDG_ADD(d_Q);
   MMDG_ADD(d_mol_shell0); MMDG_ADD(d_screen); MMDG_ADD(d_sq); MMDG_ADD(d_sqf); MMDG_ADD(d_dPf); MMDG_ADD(d_Dsh);
   MMDG_ADD(d_counters); MMDG_ADD(d_q64); MMDG_ADD(d_q32); MMDG_ADD(d_keyoff); MMDG_ADD(d_keyw); MMDG_ADD(d_qn); MMDG_ADD(d_work);
-  MMDG_ADD(d_pair_owner); MMDG_ADD(d_pair_canon);
+  MMDG_ADD(d_pair_owner); MMDG_ADD(d_pair_canon); MMDG_ADD(d_grad);
   for (int c = 0; c < kNumPairClasses; ++c) {
     MMDG_ADD(d_cls[c]); MMDG_ADD(d_cls_moff[c]); MMDG_ADD(d_gslot[c]);
   }
@@ -1852,6 +1860,9 @@ extern "C" int mmdg_set_tile(mmdg_context* h, int cls, int block_threads, int it
 // ------------------------------------------------------------------ nuclear gradient
 #include "grad.cuh"
 
+// a context keeps its gradient workspace from one geometry step to the next up to this size
+static const size_t kGradKeepBytes = size_t(64) << 20;
+
 extern "C" int mmdg_rhf_gradient(mmdg_context* h, const double* P, const double* W, int natom,
                                  const double* atom_xyz, const double* atom_Z, const int* shell_atom, double qtol,
                                  double* grad, void* stream) {
@@ -1861,16 +1872,112 @@ extern "C" int mmdg_rhf_gradient(mmdg_context* h, const double* P, const double*
   if (h->nmol != 1) return fail(MMDG_E_ARG, "mmdg_rhf_gradient: one molecule per context");
   for (int s = 0; s < h->nshell; ++s)
     if (shell_atom[s] < 0 || shell_atom[s] >= natom) return fail(MMDG_E_ARG, "mmdg_rhf_gradient: shell_atom out of range");
+  if (!(qtol >= 0.0)) return fail(MMDG_E_ARG, "mmdg_rhf_gradient: qtol must be >= 0");
   DeviceGuard dgd(h->device);
   cudaStream_t st = (cudaStream_t)stream;
-  DevBuf<double> dxyz, dZ, dg;
-  DevBuf<int> dsa;
-  if (dxyz.upload(std::vector<double>(atom_xyz, atom_xyz + 3 * natom)) != cudaSuccess ||
-      dZ.upload(std::vector<double>(atom_Z, atom_Z + natom)) != cudaSuccess ||
-      dsa.upload(std::vector<int>(shell_atom, shell_atom + h->nshell)) != cudaSuccess ||
-      dg.alloc(3 * (size_t)natom) != cudaSuccess)
+  std::lock_guard<std::mutex> lock(h->grad_mu);
+  // ---- primitive pairs: all but those whose Gaussian factor exp(-mu |AB|^2) is below
+  // e^-130 (1e-56: nothing of them reaches a double)
+  std::vector<float> Q(h->npair, 0.f);
+  if (qtol > 0.0) {
+    CUDA_TRY(cudaMemcpyAsync(Q.data(), h->d_Q.p, sizeof(float) * h->npair, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+  }
+  std::vector<int> prb(h->npair), prc(h->npair), pnnz(h->npair), pp_pair, pp_index;
+  std::vector<long long> eoff(h->npair);
+  std::vector<std::vector<int>> lists(kNumPairClasses);
+  long long ne = 0;
+  for (int p = 0; p < h->npair; ++p) {
+    const int sa = h->pa[p], sb = h->pb[p], Ka = h->shell_K[sa], Kb = h->shell_K[sb];
+    double r2 = 0.0;
+    for (int x = 0; x < 3; ++x) {
+      const double d = h->shell_center[3 * sa + x] - h->shell_center[3 * sb + x];
+      r2 += d * d;
+    }
+    prb[p] = (int)pp_pair.size();
+    for (int ka = 0; ka < Ka; ++ka)
+      for (int kb = 0; kb < Kb; ++kb) {
+        const double ea = h->prim_exp[h->shell_poff[sa] + ka], eb = h->prim_exp[h->shell_poff[sb] + kb];
+        if (ea * eb / (ea + eb) * r2 > 130.0) continue;
+        pp_pair.push_back(p);
+        pp_index.push_back(ka * Kb + kb);
+      }
+    prc[p] = (int)pp_pair.size() - prb[p];
+    pnnz[p] = nnz_pair(h->shell_L[sa], h->shell_L[sb]);
+    eoff[p] = ne;
+    ne += (long long)prc[p] * pnnz[p];
+    if (prc[p]) lists[h->pcls[p]].push_back(p);
+  }
+  const size_t npp = pp_pair.size();
+  if (npp > 0x7fffffffULL) return fail(MMDG_E_ARG, "mmdg_rhf_gradient: too many primitive pairs");
+  GradList gl[kNumPairClasses];
+  std::vector<int> all;
+  for (int c = 0; c < kNumPairClasses; ++c) {
+    std::vector<int>& v = lists[c];
+    std::stable_sort(v.begin(), v.end(), [&](int x, int y) { return prc[x] != prc[y] ? prc[x] < prc[y] : Q[x] > Q[y]; });
+    std::vector<int> vals;
+    std::vector<long long> freq;
+    for (int p : v) {
+      if (vals.empty() || vals.back() != prc[p]) {
+        vals.push_back(prc[p]);
+        freq.push_back(0);
+      }
+      ++freq.back();
+    }
+    const std::vector<int> grp = group_counts(vals, freq, kMaxGroups);
+    GradList& L = gl[c];
+    L.n = (int)v.size();
+    L.ngroup = vals.empty() ? 0 : grp.back() + 1;
+    for (int x = 0; x <= kMaxGroups; ++x) L.start[x] = L.n;
+    size_t at = v.size();
+    for (size_t x = vals.size(); x-- > 0;) {
+      at -= freq[x];
+      L.start[grp[x]] = (int)at;
+      if (x + 1 == vals.size() || grp[x + 1] != grp[x]) L.prims[grp[x]] = vals[x];
+    }
+    if ((long long)L.n * L.n > 0x7fffffffLL * 4) return fail(MMDG_E_ARG, "mmdg_rhf_gradient: too many shell pairs");
+    // inside a group by Q: quartets below qtol end up together
+    for (int x = 0; x < L.ngroup; ++x)
+      std::stable_sort(v.begin() + L.start[x], v.begin() + L.start[x + 1], [&](int p, int q) { return Q[p] > Q[q]; });
+    all.insert(all.end(), v.begin(), v.end());
+  }
+  // ---- one workspace: host data first (one copy), then what the kernels write
+  struct Part {
+    size_t at, bytes;
+  };
+  size_t size = 0;
+  auto part = [&](size_t bytes) {
+    const Part r{size, bytes};
+    size = (size + bytes + 255) & ~size_t(255);
+    return r;
+  };
+  const size_t np = (size_t)h->npair;
+  const Part o_xyz = part(24 * (size_t)natom), o_Z = part(8 * (size_t)natom), o_sa = part(4 * (size_t)h->nshell),
+             o_prb = part(4 * np), o_prc = part(4 * np), o_nnz = part(4 * np), o_eoff = part(8 * np),
+             o_ppp = part(4 * npp), o_ppi = part(4 * npp), o_list = part(4 * all.size());
+  const size_t host_bytes = size;
+  const Part o_pP = part(32 * npp), o_frac = part(8 * npp), o_E = part(8 * (size_t)ne), o_ER = part(24 * (size_t)ne),
+             o_grad = part(24 * (size_t)natom * kGradCopies), o_work = part(8 * kGradClasses);
+  if (h->d_grad.n < size && h->d_grad.alloc(size) != cudaSuccess) {
+    h->d_grad.release();
     return fail(MMDG_E_NOMEM, "mmdg_rhf_gradient: allocation");
-  CUDA_TRY(cudaMemsetAsync(dg.p, 0, sizeof(double) * 3 * natom, st));
+  }
+  std::vector<unsigned char> stage(host_bytes);
+  auto put = [&](const Part& o, const void* src) {
+    if (o.bytes) std::memcpy(stage.data() + o.at, src, o.bytes);
+  };
+  put(o_xyz, atom_xyz);
+  put(o_Z, atom_Z);
+  put(o_sa, shell_atom);
+  put(o_prb, prb.data());
+  put(o_prc, prc.data());
+  put(o_nnz, pnnz.data());
+  put(o_eoff, eoff.data());
+  put(o_ppp, pp_pair.data());
+  put(o_ppi, pp_index.data());
+  put(o_list, all.data());
+  unsigned char* ws = h->d_grad.p;
+  CUDA_TRY(cudaMemcpyAsync(ws, stage.data(), host_bytes, cudaMemcpyHostToDevice, st));
   GradArgs a;
   a.npair = h->npair;
   a.pa = h->d_pa.p;
@@ -1879,24 +1986,45 @@ extern "C" int mmdg_rhf_gradient(mmdg_context* h, const double* P, const double*
   a.nprim = h->d_nprim.p;
   a.poff = h->d_poff.p;
   a.func = h->d_func.p;
-  a.shell_atom = dsa.p;
+  a.shell_atom = (const int*)(ws + o_sa.at);
   a.center = h->d_center.p;
   a.exps = h->d_exp.p;
   a.coefs = h->d_coef.p;
-  if (!(qtol >= 0.0)) return fail(MMDG_E_ARG, "mmdg_rhf_gradient: qtol must be >= 0");
+  a.nprimpair = (int)npp;
+  a.prb = (const int*)(ws + o_prb.at);
+  a.prc = (const int*)(ws + o_prc.at);
+  a.pair_nnz = (const int*)(ws + o_nnz.at);
+  a.pp_pair = (const int*)(ws + o_ppp.at);
+  a.pp_index = (const int*)(ws + o_ppi.at);
+  a.eoff = (const long long*)(ws + o_eoff.at);
+  a.pP = (double4_32a*)(ws + o_pP.at);
+  a.frac = (double*)(ws + o_frac.at);
+  a.E64 = (double*)(ws + o_E.at);
+  a.ER = (double*)(ws + o_ER.at);
   a.Qpair = qtol > 0.0 ? h->d_Q.p : nullptr;
   a.qtol = qtol;
+  for (int x = 0; x < 10; ++x) a.small[x] = x;
   a.natom = natom;
-  a.xyz = dxyz.p;
-  a.Z = dZ.p;
+  a.xyz = (const double*)(ws + o_xyz.at);
+  a.Z = (const double*)(ws + o_Z.at);
   a.P = P;
   a.W = W;
   a.N = h->mol_n[0];
-  a.grad = dg.p;
-  CUDA_TRY(mmdg_launch_rhf_gradient(a, st));
+  a.grad = (double*)(ws + o_grad.at);
+  a.work = (unsigned long long*)(ws + o_work.at);
+  Geometry geo = h->geom();
+  geo.pP = a.pP;
+  geo.E64 = a.E64;
+  int first = 0;
+  for (int c = 0; c < kNumPairClasses; ++c) {
+    gl[c].list = (const int*)(ws + o_list.at) + first;
+    first += gl[c].n;
+  }
+  CUDA_TRY(mmdg_launch_rhf_gradient(a, geo, gl, h->nstreams, h->side, h->fork_ev, h->join_ev, st));
   std::vector<double> g(3 * (size_t)natom);
-  CUDA_TRY(cudaMemcpyAsync(g.data(), dg.p, sizeof(double) * 3 * natom, cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaMemcpyAsync(g.data(), a.grad, sizeof(double) * 3 * natom, cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
+  if (h->d_grad.n > kGradKeepBytes) h->d_grad.release();
   // nuclear repulsion: d/dR_A sum_{B<C} Z_B Z_C / R_BC (mmd/forces.py:50-58)
   for (int A = 0; A < natom; ++A)
     for (int B = 0; B < natom; ++B) {

@@ -164,7 +164,7 @@ constexpr float kLanePrims = 4.0f;
 
 template <class CountF, class WeightF>
 __device__ __forceinline__ void plan_buckets(BucketPlan& p, int nkeys, int nchunk, long long nthreads, CountF count,
-                                             WeightF weight) {
+                                             WeightF weight, int most = 5) {
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     float W = 0.f;
@@ -179,7 +179,7 @@ __device__ __forceinline__ void plan_buckets(BucketPlan& p, int nkeys, int nchun
       if (x < nkeys) {
         const unsigned c = count(nkeys - 1 - x);
         const float w = float(weight(nkeys - 1 - x));
-        while (lg < 5 && w > share * float(1 << lg)) ++lg;
+        while (lg < most && w > share * float(1 << lg)) ++lg;
         len = ((c << lg) + 31u) & ~31u;
       }
       unsigned end = len;
@@ -340,6 +340,30 @@ struct TensorBuckets {
   int bw[kMaxGroups], kw[kMaxGroups];
 };
 
+// quartets of bucket k
+__device__ __forceinline__ unsigned bucket_quartets(const TensorBuckets& tb, int same, int k) {
+  const int gb = k / tb.nkg, gk = k - gb * tb.nkg;
+  const unsigned a = tb.bstart[gb + 1] - tb.bstart[gb], b = tb.kstart[gk + 1] - tb.kstart[gk];
+  return !same || gk < gb ? a * b : (gk == gb ? a * (a + 1) / 2 : 0u);
+}
+
+// bra and ket list slot of a bucket's quartet
+__device__ __forceinline__ void bucket_slot(const TensorBuckets& tb, int same, int key, unsigned slot, int& ib, int& jk) {
+  const int gb = key / tb.nkg, gk = key - gb * tb.nkg;
+  if (same && gb == gk) {  // slot = ib (ib + 1) / 2 + jk
+    ib = (int)((sqrtf(8.0f * float(slot) + 1.0f) - 1.0f) * 0.5f);
+    while ((long long)ib * (ib + 1) / 2 > (long long)slot) --ib;
+    while ((long long)(ib + 1) * (ib + 2) / 2 <= (long long)slot) ++ib;
+    jk = (int)((long long)slot - (long long)ib * (ib + 1) / 2);
+  } else {
+    const unsigned b = tb.kstart[gk + 1] - tb.kstart[gk];
+    ib = (int)(slot / b);
+    jk = (int)(slot - (unsigned)ib * b);
+  }
+  ib += tb.bstart[gb];
+  jk += tb.kstart[gk];
+}
+
 // Every ERI of the class into the tensor, 1 to 32 lanes per (quartet, ket chunk) as in
 // k_fock, persistent over the buckets.  (One thread per quartet: N = 75 10.6 ms, its 21
 // launches each as long as their heaviest quartet; with groups 2.2 ms.)
@@ -347,12 +371,8 @@ template <class MD>
 __global__ void __launch_bounds__(kThreads) k_tensor(Geometry g, TensorArgs t, ClassLaunch cl, TensorBuckets tb) {
   __shared__ BucketPlan plan;
   const int nkeys = tb.nbg * tb.nkg;
-  auto count = [&](int k) -> unsigned {
-    const int gb = k / tb.nkg, gk = k - gb * tb.nkg;
-    const unsigned a = tb.bstart[gb + 1] - tb.bstart[gb], b = tb.kstart[gk + 1] - tb.kstart[gk];
-    return !cl.same || gk < gb ? a * b : (gk == gb ? a * (a + 1) / 2 : 0u);
-  };
-  plan_buckets(plan, nkeys, MD::NCHUNK, (long long)gridDim.x * kThreads, count,
+  plan_buckets(plan, nkeys, MD::NCHUNK, (long long)gridDim.x * kThreads,
+               [&](int k) { return bucket_quartets(tb, cl.same, k); },
                [&](int k) { return tb.bw[k / tb.nkg] * tb.kw[k % tb.nkg]; });
   const unsigned n = plan.pre[nkeys];
   const long long total = (long long)n * MD::NCHUNK, stride = (long long)gridDim.x * kThreads;
@@ -367,20 +387,10 @@ __global__ void __launch_bounds__(kThreads) k_tensor(Geometry g, TensorArgs t, C
     while (r >= plan.pre[x + 1]) ++x;
     const int lg = plan.lg[x], key = nkeys - 1 - x;
     const unsigned slot = (r - plan.pre[x]) >> lg;
-    if (slot >= count(key)) continue;
-    const int gb = key / tb.nkg, gk = key - gb * tb.nkg;
+    if (slot >= bucket_quartets(tb, cl.same, key)) continue;
     int ib, jk;
-    if (cl.same && gb == gk) {  // slot = ib (ib + 1) / 2 + jk
-      ib = (int)((sqrtf(8.0f * float(slot) + 1.0f) - 1.0f) * 0.5f);
-      while ((long long)ib * (ib + 1) / 2 > (long long)slot) --ib;
-      while ((long long)(ib + 1) * (ib + 2) / 2 <= (long long)slot) ++ib;
-      jk = (int)((long long)slot - (long long)ib * (ib + 1) / 2);
-    } else {
-      const unsigned b = tb.kstart[gk + 1] - tb.kstart[gk];
-      ib = (int)(slot / b);
-      jk = (int)(slot - (unsigned)ib * b);
-    }
-    const int bp = __ldg(cl.bra + tb.bstart[gb] + ib), kp = __ldg(cl.ket + tb.kstart[gk] + jk);
+    bucket_slot(tb, cl.same, key, slot, ib, jk);
+    const int bp = __ldg(cl.bra + ib), kp = __ldg(cl.ket + jk);
     const int sa = __ldg(g.pa + bp), sb = __ldg(g.pb + bp), sc = __ldg(g.pa + kp), sd = __ldg(g.pb + kp);
     Ctx<double> c = make_ctx<MD, double>(g, bp, kp, rs);
     c.chunk = MD::NCHUNK > 1 ? chunk : -1;
