@@ -1334,27 +1334,99 @@ extern "C" int mmdg_set_screen(mmdg_context* h, const double* screen, long long 
   return MMDG_OK;
 }
 
-// J_pq = sum_rs (pq|rs) P_sr,  K_pq = sum_rs (ps|qr) P_sr   (mmd/scf.py:97-98)
-// one warp per (p,q); lanes stride over r,s
-__global__ void k_jk_dense(const double* T, const double* P, double* J, double* K, long long N) {
-  const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+// J_pq = sum_rs (pq|rs) P_sr,  K_pq = sum_rs (ps|qr) P_sr   (mmd/scf.py:97-98), for any
+// tensor T and matrix P.  Bound by the FP64 pipe: two FMAs per 8-byte element are 0.32 ms
+// at N = 100 (a read of the tensor is 0.12 ms, so reading it once for J and once for K is
+// covered).  Both sums walk the tensor in memory order, with no sum over lanes inside the
+// loop and no atomics:
+//   J blocks take kJRows consecutive rows pq; a thread keeps one accumulator per row and
+//     reads each P_sr once for all of them;
+//   K blocks take one p and a run of rows q, their (q, r) positions flattened over the
+//     threads (kKPos each, so N need not be a multiple of 32), one accumulator per position
+//     over the loop over s; the positions of a row are added up at the end.
+// One warp per (p, q) with lanes over (r, s), the exchange at a stride of N^2 elements, took
+// 749 us at N = 100 (42 at N = 50), this form 369 (34).  Measured beside it: 4 or 16 rows
+// per J block 379 / 370, 4 positions per thread 375 and 48 at N = 50.
+constexpr int kJKThreads = 256, kJRows = 8, kKPos = 2;
+
+__global__ void __launch_bounds__(kJKThreads) k_jk_dense(const double* __restrict__ T, const double* __restrict__ P,
+                                                         double* __restrict__ J, double* __restrict__ K, int N, int nj,
+                                                         int qrows, int qblocks) {
+  __shared__ double sum[kJKThreads * kKPos];
+  const long long NN = (long long)N * N;
+  if ((int)blockIdx.x < nj) {
+    const long long row0 = (long long)blockIdx.x * kJRows;
+    const int rows = (int)min((long long)kJRows, NN - row0);
+    const double* __restrict__ t = T + row0 * NN;
+    double acc[kJRows];
+#pragma unroll
+    for (int x = 0; x < kJRows; ++x) acc[x] = 0.0;
+    if (rows == kJRows) {
+      for (long long e = threadIdx.x; e < NN; e += kJKThreads) {
+        const int r = (int)(e / N), s = (int)(e - (long long)r * N);
+        const double psr = __ldg(P + (long long)s * N + r);
+#pragma unroll
+        for (int x = 0; x < kJRows; ++x) acc[x] = fma(__ldcs(t + x * NN + e), psr, acc[x]);
+      }
+    } else {
+      for (long long e = threadIdx.x; e < NN; e += kJKThreads) {
+        const int r = (int)(e / N), s = (int)(e - (long long)r * N);
+        const double psr = __ldg(P + (long long)s * N + r);
+        for (int x = 0; x < kJRows; ++x)
+          if (x < rows) acc[x] = fma(__ldcs(t + x * NN + e), psr, acc[x]);
+      }
+    }
+    // rows x lanes -> one row per lane: each step halves the rows a lane still holds
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int h = kJRows / 2, o = 16; h > 0; h >>= 1, o >>= 1)
+#pragma unroll
+      for (int x = 0; x < h; ++x) {
+        const bool up = lane & o;
+        const double give = up ? acc[x] : acc[x + h], keep = up ? acc[x + h] : acc[x];
+        acc[x] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    double v = acc[0];
+#pragma unroll
+    for (int o = 32 / kJRows / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane % (32 / kJRows) == 0) sum[warp * kJRows + lane / (32 / kJRows)] = v;
+    __syncthreads();
+    if ((int)threadIdx.x < rows) {
+      double s = 0.0;
+      for (int w = 0; w < kJKThreads / 32; ++w) s += sum[w * kJRows + threadIdx.x];
+      J[row0 + threadIdx.x] = s;
+    }
+    return;
+  }
+  const int b = (int)blockIdx.x - nj, p = b / qblocks, q0 = (b - p * qblocks) * qrows;
+  const int nq = min(qrows, N - q0), npos = nq * N;
+  const double* __restrict__ t = T + (long long)p * NN * N + (long long)q0 * N;  // + s N^2 + position
+  double acc[kKPos];
+  int r[kKPos];
+#pragma unroll
+  for (int x = 0; x < kKPos; ++x) {
+    acc[x] = 0.0;
+    r[x] = (int)(threadIdx.x + x * kJKThreads) % N;
+  }
+#pragma unroll 4
+  for (int s = 0; s < N; ++s) {
+    const double* __restrict__ ts = t + s * NN;
+    const double* __restrict__ ps = P + (long long)s * N;
+#pragma unroll
+    for (int x = 0; x < kKPos; ++x) {
+      const int pos = threadIdx.x + x * kJKThreads;
+      if (pos < npos) acc[x] = fma(__ldcs(ts + pos), __ldg(ps + r[x]), acc[x]);
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < kKPos; ++x) sum[threadIdx.x + x * kJKThreads] = acc[x];
+  __syncthreads();
   const int lane = threadIdx.x & 31;
-  if (w >= N * N) return;
-  const long long p = w / N, q = w % N;
-  double j = 0.0, k = 0.0;
-  for (long long x = lane; x < N * N; x += 32) {
-    const long long r = x / N, s = x % N;
-    const double psr = P[s * N + r];
-    j = fma(T[((p * N + q) * N + r) * N + s], psr, j);
-    k = fma(T[((p * N + s) * N + q) * N + r], psr, k);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    j += __shfl_xor_sync(0xffffffffu, j, o);
-    k += __shfl_xor_sync(0xffffffffu, k, o);
-  }
-  if (lane == 0) {
-    J[p * N + q] = j;
-    K[p * N + q] = k;
+  for (int q = threadIdx.x >> 5; q < nq; q += kJKThreads / 32) {
+    double v = 0.0;
+    for (int x = lane; x < N; x += 32) v += sum[q * N + x];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) K[(long long)p * N + q0 + q] = v;
   }
 }
 
@@ -1362,8 +1434,11 @@ extern "C" int mmdg_jk_dense(mmdg_context* h, long long N, const double* T, cons
                              void* stream) {
   if (!h || !T || !P || !J || !K || N <= 0) return fail(MMDG_E_ARG, "mmdg_jk_dense: bad argument");
   DeviceGuard dg(h->device);
-  const long long warps = N * N;
-  k_jk_dense<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(T, P, J, K, N);
+  // (a K block holds at least one row: N^4 elements of a larger N are past any memory)
+  if (N > kJKThreads * kKPos) return fail(MMDG_E_ARG, "mmdg_jk_dense: N above 512");
+  const int n = (int)N, nj = (int)((N * N + kJRows - 1) / kJRows);
+  const int qrows = std::min(n, kJKThreads * kKPos / n), qblocks = (n + qrows - 1) / qrows;
+  k_jk_dense<<<nj + n * qblocks, kJKThreads, 0, (cudaStream_t)stream>>>(T, P, J, K, n, nj, qrows, qblocks);
   CUDA_TRY(cudaGetLastError());
   return MMDG_OK;
 }
