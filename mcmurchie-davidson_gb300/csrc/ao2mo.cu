@@ -8,11 +8,23 @@
 // order: pqrs -> Spqr -> RSpq -> QRSp -> PQRS.  Each call is a GEMM
 // out (N x N^3) = C^T (N x N) . in^T (N x N^3) in FP64: 64 x 64 output tiles per
 // 256-thread block, 4 x 4 outputs per thread, the K dimension staged through shared
-// memory 16 at a time.  An FP64 warp instruction holds the FP64 pipe of its
+// memory 16 at a time (k_quarter; N > 128).  An FP64 warp instruction holds the FP64 pipe of its
 // sub-partition for ~64 cycles on this GPU, so the eight shared-memory loads around
 // a thread's 16 independent FMAs per k step cost nothing; the 16 accumulators keep
 // the pipe fed.
+//
+// Up to N = 128 the product runs on the tensor cores instead (k_quarter_tc), exactly
+// up to a rounding far below a double's: every row of the tensor and every column of C is
+// scaled by a power of two and cut into eight signed 8-bit digits (62 bits), digits are
+// exact BF16 numbers, and the digit products with i + j = d, d = 0..7 (36 of 64), are
+// summed by tcgen05.mma in one FP32 accumulator per d: at most 8 x 128 products of at
+// most 2^14, so every sum is an integer of at most 2^24 and exact.  The eight integers
+// are put together in fixed point and rounded once.  Left out are digit products below
+// 2^-62 of (row maximum) x (column maximum).  (Split-operand products after K. Ozaki,
+// T. Ogita, S. Oishi and S. M. Rump, Numer. Algorithms 59, 95-118, 2012.)
 #include <cuda_runtime.h>
+
+#include <stdint.h>
 
 #include "../../include/mmdg.h"
 
@@ -75,7 +87,318 @@ __global__ void __launch_bounds__(256) k_quarter(const double* __restrict__ in, 
   }
 }
 
+
+// ------------------------------------------------------------------ tensor-core form
+constexpr int kTcThreads = 256;
+constexpr int kTcRows = 128;                        // rows m of the tensor per tile (MMA M)
+constexpr int kTcCols = 32;                         // new indices S per block (MMA N)
+constexpr int kTcDigits = 8;
+constexpr int kTcStage = kTcRows * 16 * 2;          // bytes of one digit of a 16-wide k step
+constexpr int kTcTmem = kTcDigits * kTcCols;        // accumulator columns
+constexpr int kTcRawStride = 17;                    // doubles per row of the raw stage (16 + 1: no bank conflict)
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// K-major operand without swizzle: 8 x 16-byte core matrices of 128 contiguous bytes, `lbo`
+// bytes apart along k and 128 bytes apart along the rows
+__device__ __forceinline__ uint64_t operand(uint32_t addr, uint32_t lbo) {
+  return (uint64_t)((addr >> 4) & 0x3fff) | (uint64_t)((lbo >> 4) & 0x3fff) << 16 | (uint64_t)(128 >> 4) << 32 |
+         (uint64_t)1 << 46;
+}
+__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t add) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(add)
+      : "memory");
+}
+// waits for the barrier's phase; false when it did not come (never expected: then the
+// block's outputs become NaN instead of the kernel spinning on)
+__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t phase) {
+  for (int i = 0; i < (1 << 22); ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(phase)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void tmem_load8(uint32_t addr, uint32_t* v) {
+  // (the wait in the same statement: nothing that uses the registers can move before it)
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+               "tcgen05.wait::ld.sync.aligned;\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(addr));
+}
+
+// x 2^(1084 - emax) as a fixed-point number (|.| < 2^62, truncated), plus 128 in every byte:
+// byte 7 - i minus 128 is then its signed digit i.  emax: the largest exponent field of the
+// row (at least 1).
+__device__ __forceinline__ uint64_t fixed_digits(double x, int emax) {
+  const uint64_t b = (uint64_t)__double_as_longlong(x);
+  const int e = (int)(b >> 52) & 0x7ff, ee = e > 1 ? e : 1;
+  const uint64_t m = (b & 0xfffffffffffffULL) | (e ? 1ULL << 52 : 0ULL);
+  uint64_t v = (m << 9) >> min(emax - ee, 63);
+  if ((int64_t)b < 0) v = 0ULL - v;
+  return v + 0x8080808080808080ULL;
+}
+// digit i of two fixed-point numbers as a pair of BF16 (the first in the low half): the byte
+// placed into 2^23's mantissa, 2^23 + 128 subtracted (exact), the upper halves packed
+__device__ __forceinline__ uint32_t digit_pair(uint64_t u, uint64_t v, int i) {
+  const int byte = 7 - i;
+  const uint32_t us = byte >= 4 ? (uint32_t)(u >> 32) : (uint32_t)u, vs = byte >= 4 ? (uint32_t)(v >> 32) : (uint32_t)v;
+  const uint32_t sel = 0x7440u | (uint32_t)(byte & 3);
+  const float f = __uint_as_float(__byte_perm(us, 0x4B000000u, sel)) - 8388736.0f;
+  const float g = __uint_as_float(__byte_perm(vs, 0x4B000000u, sel)) - 8388736.0f;
+  return __byte_perm(__float_as_uint(f), __float_as_uint(g), 0x7632u);
+}
+// eight consecutive k of one row: their digits as one 16-byte core-matrix row per digit
+__device__ __forceinline__ void store_digits(const double* x, int emax, unsigned char* at, int digit_bytes) {
+  uint32_t w[kTcDigits][4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const uint64_t u = fixed_digits(x[2 * p], emax), v = fixed_digits(x[2 * p + 1], emax);
+#pragma unroll
+    for (int i = 0; i < kTcDigits; ++i) w[i][p] = digit_pair(u, v, i);
+  }
+#pragma unroll
+  for (int i = 0; i < kTcDigits; ++i)
+    *reinterpret_cast<uint4*>(at + i * digit_bytes) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+}
+
+// the rare cases, kept out of line: a result outside the normal doubles, and a row or column
+// with an infinity or NaN (as plain arithmetic has it)
+__device__ __noinline__ double scaled(uint64_t mant, int e) { return ldexp((double)mant, e); }
+__device__ __noinline__ double plain_dot(const double* __restrict__ row, const double* __restrict__ C, int N) {
+  double v = 0.0;
+  for (int k = 0; k < N; ++k) v = fma(__ldg(row + k), __ldg(C + (long long)k * N), v);
+  return v;
+}
+
+// sum_d acc_d 256^(7-d) 2^scale as a double, rounded to nearest, without a branch (eight of
+// them interleave); outside the normal doubles `far` is set, and the value is (-1)^neg mant 2^e
+__device__ __forceinline__ double assemble(const uint32_t (*acc)[8], int col, int scale, bool& far, bool& neg,
+                                           uint64_t& mant, int& e) {
+  int a[kTcDigits];
+#pragma unroll
+  for (int d = 0; d < kTcDigits; ++d) a[d] = __float2int_rn(__uint_as_float(acc[d][col]));
+  long long hi = (long long)a[0] * (1 << 24) + ((long long)a[1] * (1 << 16) + ((long long)a[2] * (1 << 8) + a[3]));
+  const long long lo = (long long)a[4] * (1 << 24) + ((long long)a[5] * (1 << 16) + ((long long)a[6] * (1 << 8) + a[7]));
+  hi += lo >> 32;  // value = hi 2^32 + (low 32 bits of lo)
+  neg = hi < 0;  // magnitude of the 96-bit two's complement number
+  const uint32_t low = neg ? 0u - (uint32_t)lo : (uint32_t)lo;
+  hi = neg ? ~hi + (low == 0u) : hi;
+  const bool small = hi == 0;
+  const uint64_t h = small ? (uint64_t)low : (uint64_t)hi, rest = small ? 0ULL : (uint64_t)low << 32;
+  const int lead = __clzll((long long)h);  // 64 for zero
+  const uint64_t top = (h << (lead & 63)) | ((rest >> 1) >> (63 - (lead & 63)));  // leading one at bit 63
+  mant = (top >> 11) + ((top >> 10) & 1);                                         // 2^52 .. 2^53
+  e = (small ? 0 : 32) - lead + 11 + scale;                                       // value = mant 2^e
+  const int field = e + 1075;
+  far = h != 0 && (field <= 0 || field >= 2046);
+  const uint64_t bits = ((uint64_t)(uint32_t)(field - 1) << 52) + mant;
+  return __longlong_as_double((long long)(h == 0 ? 0ULL : (bits | (uint64_t)neg << 63)));
+}
+
+// One quarter transform.  Block (x, y): the S tile y (its digits of C stay in shared memory)
+// of the row tiles x, x + gridDim.x, ...  Per 16-wide k step the block stages the raw rows,
+// cuts them into digits and one thread issues the 36 digit products; two blocks per SM
+// (256 of the 512 TMEM columns each) overlap one's products with the other's digits.
+// Bound by the integer work around the products: of a tile's ~31,000 cycles at N = 76 (two
+// blocks per SM) about 6,600 cut digits, 7,400 put results together, 7,500 find the row
+// exponents and 6,000 stage rows; the tensor pipe is busy for 7 %.  One product of N =
+// (8 - i) NT columns per row digit i, instead of one per digit pair, took issuing them
+// from 2,400 to 150 cycles a step.  us per transform, k_quarter -> this: N = 7 86 -> 37,
+// 13 86 -> 43, 32 537 -> 77, 64 6,930 -> 926, 76 28,980 -> 2,720, 100 91,700 -> 10,400,
+// 128 219,500 -> 33,100 (FP64 arithmetic alone is 16,000 at N = 76, memory 320).
+// Prefetching the next tile into L2 was slower up to N = 76.
+__global__ void __launch_bounds__(kTcThreads, 2)
+    k_quarter_tc(const double* __restrict__ in, const double* __restrict__ C, double* __restrict__ out, int N,
+                 long long M) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  __shared__ __align__(8) uint64_t s_bar;
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_rows[2][kTcRows];  // largest exponent field of every row, this tile's and the next one's
+  __shared__ int s_col[kTcCols];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int steps = (N + 15) / 16, Kp = steps * 16;
+  const int S0 = blockIdx.y * kTcCols, cols = min(kTcCols, N - S0), NT = (cols + 15) & ~15;
+  unsigned char* const As = sm;                                          // [digit][k octet][row][16 B]
+  double* const raw = reinterpret_cast<double*>(sm + kTcDigits * kTcStage);
+  unsigned char* const Bs = sm + kTcDigits * kTcStage + sizeof(double) * kTcRawStride * kTcRows;  // [k octet][digit][S][16 B]
+  const uint32_t bar = smem_addr(&s_bar);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)),
+                 "r"(kTcTmem)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  // ---- C's digits
+  for (int n = warp; n < kTcCols; n += kTcThreads / 32) {
+    unsigned top = 0;
+    if (n < cols)
+      for (int k = lane; k < N; k += 32)
+        top = max(top, (unsigned)__double2hiint(__ldg(C + (long long)k * N + S0 + n)) & 0x7fffffffu);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) s_col[n] = max((int)(top >> 20), 1);
+  }
+  __syncthreads();
+  const uint32_t tmem = s_tmem;
+  for (int u = tid; u < NT * (Kp / 8); u += kTcThreads) {
+    const int n = u % NT, oct = u / NT;
+    double x[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = oct * 8 + j;
+      x[j] = n < cols && k < N ? __ldg(C + (long long)k * N + S0 + n) : 0.0;
+    }
+    store_digits(x, s_col[n], Bs + (oct * kTcDigits * NT + n) * 16, NT * 16);
+  }
+  // instruction descriptor: D FP32, A and B BF16, both K-major, M (N is added per product)
+  const uint32_t idesc = 1u << 4 | 1u << 7 | 1u << 10 | (uint32_t)(kTcRows >> 4) << 24;
+  uint32_t phase = 0;
+  bool good = true;
+  // largest exponent of every row of the tile at m: a warp per 16 rows, their loads in flight
+  // together (row by row this took 25,000 of a tile's 54,000 cycles)
+  auto row_exponents = [&](long long m, int* to) {
+    constexpr int R = kTcRows / 8;
+    const int rows = (int)min((long long)kTcRows, M - m) - warp * R;
+    const int* __restrict__ src = reinterpret_cast<const int*>(in + (m + warp * R) * N) + 1;  // high words
+    unsigned top[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) top[r] = 0u;
+    for (int k = lane; k < N; k += 64) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int* __restrict__ h = src + 2 * (r * N + k);
+        const unsigned u = r < rows ? (unsigned)__ldg(h) & 0x7fffffffu : 0u;
+        const unsigned w = r < rows && k + 32 < N ? (unsigned)__ldg(h + 64) & 0x7fffffffu : 0u;
+        top[r] = max(top[r], max(u, w));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const unsigned v = __reduce_max_sync(0xffffffffu, top[r]);
+      if (lane == 0) to[warp * R + r] = max((int)(v >> 20), 1);
+    }
+  };
+  const long long mstep = (long long)gridDim.x * kTcRows;
+  int buf = 0;
+  if ((long long)blockIdx.x * kTcRows < M) row_exponents((long long)blockIdx.x * kTcRows, s_rows[0]);
+  const int lr = tid >> 4, lk = tid & 15;  // raw staging: row lr + 16 x, k lk
+  const int row = tid & (kTcRows - 1), oct = tid >> 7;
+  for (long long m0 = (long long)blockIdx.x * kTcRows; m0 < M; m0 += mstep, buf ^= 1) {
+    const int rows = (int)min((long long)kTcRows, M - m0);
+    const double* __restrict__ src = in + m0 * N;
+    double nxt[8];
+#pragma unroll
+    for (int x = 0; x < 8; ++x)
+      nxt[x] = lr + 16 * x < rows && lk < N ? __ldg(src + (long long)(lr + 16 * x) * N + lk) : 0.0;
+    const int* const s_row = s_rows[buf];
+    for (int st = 0; st < steps; ++st) {
+#pragma unroll
+      for (int x = 0; x < 8; ++x) raw[(lr + 16 * x) * kTcRawStride + lk] = nxt[x];
+      if (st + 1 < steps) {
+        const int k = (st + 1) * 16 + lk;
+#pragma unroll
+        for (int x = 0; x < 8; ++x)
+          nxt[x] = lr + 16 * x < rows && k < N ? __ldg(src + (long long)(lr + 16 * x) * N + k) : 0.0;
+      }
+      __syncthreads();  // raw rows and exponents are in place
+      if (st > 0) {     // the products of the previous step have read the digits
+        good = good && wait_phase(bar, phase);
+        phase ^= 1;
+      }
+      {
+        double x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = raw[row * kTcRawStride + oct * 8 + j];
+        store_digits(x, s_row[row], As + (oct * kTcRows + row) * 16, kTcStage);
+      }
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      __syncthreads();
+      if (tid == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        // the digits of C lie one after another along N, the accumulators one after another in
+        // TMEM: digit i of the rows meets digits 0 .. 7 - i of C in one product of N =
+        // (8 - i) NT columns, added into accumulators i .. 7
+        const uint32_t a0 = smem_addr(As);
+        const uint64_t b = operand(smem_addr(Bs) + (uint32_t)(st * 2 * kTcDigits * NT * 16), (uint32_t)(kTcDigits * NT * 16));
+#pragma unroll
+        for (int i = 0; i < kTcDigits; ++i)
+          mma_bf16(tmem + (uint32_t)(i * NT), operand(a0 + i * kTcStage, kTcRows * 16), b,
+                   idesc | (uint32_t)(((kTcDigits - i) * NT) >> 3) << 17, st > 0 || i > 0 ? 1u : 0u);
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
+                     : "memory");
+      }
+    }
+    if (m0 + mstep < M) row_exponents(m0 + mstep, s_rows[buf ^ 1]);  // beside the last products
+    good = good && wait_phase(bar, phase);
+    phase ^= 1;
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    // ---- outputs: lane = row of the warp's quarter, the two warps of a quarter share the columns
+    const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * (NT / 2);
+    const int er = s_row[r];
+    for (int c = c0; c < c0 + NT / 2; c += 8) {
+      uint32_t acc[kTcDigits][8];
+#pragma unroll
+      for (int d = 0; d < kTcDigits; ++d)
+        tmem_load8(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(d * NT + c), acc[d]);
+      double v[8];
+      unsigned odd = 0;  // columns that the common path does not cover
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        const int ec = s_col[c + x];
+        bool far, neg;
+        uint64_t mant;
+        int e;
+        v[x] = assemble(acc, x, er + ec - 2168 + 56, far, neg, mant, e);
+        odd |= (far || er == 0x7ff || ec == 0x7ff ? 1u : 0u) << x;
+      }
+      if (odd) {
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+          const int ec = s_col[c + x];
+          if (!(odd >> x & 1) || c + x >= cols || r >= rows) continue;
+          bool far, neg;
+          uint64_t mant;
+          int e;
+          assemble(acc, x, er + ec - 2168 + 56, far, neg, mant, e);
+          if (er == 0x7ff || ec == 0x7ff) v[x] = plain_dot(src + (long long)r * N, C + S0 + c + x, N);
+          else v[x] = neg ? -scaled(mant, e) : scaled(mant, e);
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < 8; ++x)
+        if (c + x < cols && r < rows)
+          out[(long long)(S0 + c + x) * M + m0 + r] = good ? v[x] : __longlong_as_double(0x7ff8000000000000LL);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();  // accumulators, exponents and raw rows are free again
+  }
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTcTmem));
+}
+
+// at least a third of an SM's shared memory, so that two blocks (2 x 256 TMEM columns), never
+// three, share an SM
+inline size_t tc_smem(int N) {
+  const int Kp = (N + 15) / 16 * 16, NT = N < kTcCols ? (N + 15) / 16 * 16 : kTcCols;
+  const size_t need = (size_t)kTcDigits * kTcStage + sizeof(double) * kTcRawStride * kTcRows + (size_t)kTcDigits * Kp * NT * 2;
+  return need < 80 * 1024 ? 80 * 1024 : need;
+}
+
 }  // namespace
+
+// largest N of the tensor-core form: its sums are exact up to here
+static const long long kTcMax = 128;
 
 extern "C" int mmdg_ao2mo(long long N, const double* C, const double* eri_in, double* eri_out, double* work,
                           void* stream) {
@@ -89,8 +412,23 @@ extern "C" int mmdg_ao2mo(long long N, const double* C, const double* eri_in, do
   const dim3 grid((unsigned)((M + TMv - 1) / TMv), (unsigned)((N + TS - 1) / TS));
   const double* src[4] = {eri_in, work, eri_out, work};
   double* dst[4] = {work, eri_out, work, eri_out};
+  const bool tc = N <= kTcMax;
+  const size_t smem = tc ? tc_smem((int)N) : 0;
+  dim3 tgrid;
+  if (tc) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_quarter_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return mmdg_internal_fail(MMDG_E_CUDA, cudaGetErrorString(e));
+    const long long tiles = (M + kTcRows - 1) / kTcRows, per = smem <= 111 * 1024 ? 2 : 1;
+    tgrid.y = (unsigned)((N + kTcCols - 1) / kTcCols);
+    const long long want = per * sms / tgrid.y;
+    tgrid.x = (unsigned)(want < 1 ? 1 : (want < tiles ? want : tiles));
+  }
   for (int q = 0; q < 4; ++q) {
-    k_quarter<<<grid, 256, 0, st>>>(src[q], C, dst[q], (int)N, M);
+    if (tc) k_quarter_tc<<<tgrid, kTcThreads, smem, st>>>(src[q], C, dst[q], (int)N, M);
+    else k_quarter<<<grid, 256, 0, st>>>(src[q], C, dst[q], (int)N, M);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return mmdg_internal_fail(MMDG_E_CUDA, cudaGetErrorString(e));
   }
