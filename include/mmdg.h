@@ -224,6 +224,11 @@ int mmdg_fock_graph(mmdg_context* ctx, const double* dP, double* G, double tol, 
  *   mmdg_mlp_mse       dY = 2 (Y - T) mask / count; *loss += sum ((Y - T) mask)^2 / count
  *   mmdg_mlp_adam      Adam step on FP32 master weights, refreshing their BF16 copy
  *   mmdg_mlp_to_bf16   BF16 copy of FP32 weights
+ * and fused forms of a layer's steps:
+ *   mmdg_mlp_linear      Z = X W^T + b, Y = silu(Z) (silu != 0) or Y = Z
+ *   mmdg_mlp_back        dZp = (dZ W) * silu'(Zp) (or dZ W), db[c] = sum_r dZp[r, c]
+ *   mmdg_mlp_mse_masked  mmdg_mlp_mse with count = max(sum of the mask, 1) found on the device
+ *   mmdg_mlp_adam_many   mmdg_mlp_adam of several tensors (host arrays of their pointers)
  */
 int mmdg_mlp_gemm(int M, int N, int K, const void* A, int lda, int ta, int a_bf16, const void* B, int ldb, int tb,
                   int b_bf16, float* C, int ldc, float beta, void* stream);
@@ -235,6 +240,15 @@ int mmdg_mlp_mse(const float* Y, const float* T, const float* mask, float* dY, d
 int mmdg_mlp_adam(float* w, void* w_bf16, const float* g, float* m, float* v, long long n, float lr, float b1,
                   float b2, float eps, int step, void* stream);
 int mmdg_mlp_to_bf16(const float* w, void* w_bf16, long long n, void* stream);
+int mmdg_mlp_linear(long long rows, int out, int in, const float* X, const void* W, const float* b, float* Z, float* Y,
+                    int silu, void* stream);
+int mmdg_mlp_back(long long rows, int out, int in, const float* dZ, const void* W, const float* Zp, float* dZp,
+                  float* db, int silu, void* stream);
+int mmdg_mlp_mse_masked(const float* Y, const float* T, const float* mask, float* dY, double* loss, double* count,
+                        long long n, void* stream);
+int mmdg_mlp_adam_many(int count, float* const* w, void* const* w_bf16, const float* const* g, float* const* m,
+                       float* const* v, const long long* n, float lr, float b1, float b2, float eps, int step,
+                       void* stream);
 
 /* AO -> MO transform of an ERI tensor (mmd/postscf.py:26-27, four einsums with the MO
  * coefficients): eri_out[P,Q,R,S] = sum_pqrs C[p,P] C[q,Q] C[r,R] C[s,S] eri_in[p,q,r,s].

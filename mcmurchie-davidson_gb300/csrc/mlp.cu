@@ -4,8 +4,8 @@
 // The network maps atom-pair features to density-matrix blocks (the SCF's initial
 // guess; the reference starts from P = 0, mmd/scf.py:15,23-24).  Sizes are tiny
 // (~100 k parameters, ~1 M training pairs), so the GEMMs are shared-memory tiled
-// FP32 FMA kernels reading BF16 weights; they are a few ms per epoch and not a hot
-// path of the ERI work.
+// FP32 FMA kernels reading BF16 weights (activations and sums stay FP32, as the tensor
+// cores' FP32 sums truncate), with the layers' elementwise work in their epilogues.
 //
 //   gemm:   C[M,N] (+)= op(A)[M,K] op(B)[K,N], A/B in FP32 or BF16, C in FP32
 //   act:    Y = silu(Z + b) (stores Z + b for the backward), or identity
@@ -21,7 +21,8 @@
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16;
+constexpr int TM = 128, TN = 64, TK = 16;
+constexpr int TT = TM * TN / 32;  // threads of a GEMM block, 8 x 4 outputs each
 
 template <typename T>
 __device__ __forceinline__ float ld(const T* p, long long i);
@@ -32,61 +33,146 @@ __device__ __forceinline__ float ld<__nv_bfloat16>(const __nv_bfloat16* p, long 
   return __bfloat162float(p[i]);
 }
 
-// C = alpha * op(A) op(B) + beta * C;  op(A): ta ? A^T (A stored K x M) : A (M x K)
-template <typename TA, typename TB>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const TA* A, int lda, int ta, const TB* B, int ldb,
-                                              int tb, float* C, int ldc, float beta) {
-  __shared__ float As[TK][TM + 1];
-  __shared__ float Bs[TK][TN + 1];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+// What a GEMM does with its sums.
+enum Epilogue {
+  kStore,   // C (+)= sums (atomics when K is split over blockIdx.z)
+  kLinear,  // C = Z = sums + bias (row broadcast), Y = silu(Z) or Z
+  kActGrad  // C = sums * silu'(Zp), db[n] += its column sums (db zeroed by the launcher)
+};
+struct EpilogueArgs {
+  const float* bias = nullptr;
+  float* Y = nullptr;
+  const float* Zp = nullptr;
+  float* db = nullptr;
+  int silu = 0;
+};
+
+__device__ __forceinline__ float silu_of(float z) { return z / (1.f + expf(-z)); }
+__device__ __forceinline__ float silu_grad(float z) {
+  const float s = 1.f / (1.f + expf(-z));
+  return s * (1.f + z * (1.f - s));
+}
+
+// op(A) op(B);  op(A): ta ? A^T (A stored K x M) : A (M x K), likewise B.  128 x 64 tiles, 8 x 4
+// outputs per thread read as float4 from shared memory (three 16-byte loads per 32 FMAs),
+// the next K stage in registers meanwhile.  Bound by FP32 issue (FMAs and the fetches'
+// index work) and, at the network's sizes, by the last wave: 256 tiles of an 8192 x 256
+// layer on 152 SMs.  With 64 x 64 tiles, 4 x 4 outputs and scalar shared loads the eight
+// GEMMs of a training step of 8192 rows took 840 us (7.7 TFLOP/s), now 300 (22).  Measured
+// per step: 128 x 64 tiles 363 us, 64 x 64 489, their K stage 8 or 32 deep 393 / 439.
+template <typename TA, typename TB, int EPI>
+__global__ void __launch_bounds__(TT) k_gemm(int M, int N, int K, const TA* __restrict__ A, int lda, int ta,
+                                              const TB* __restrict__ B, int ldb, int tb, float* __restrict__ C, int ldc,
+                                              float beta, EpilogueArgs ep) {
+  __shared__ __align__(16) float As[2][TK][TM + 4];
+  __shared__ __align__(16) float Bs[2][TK][TN + 4];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
   // split K over blockIdx.z (the weight gradients: M x N small, K = batch rows)
-  const int kspan = (K + gridDim.z - 1) / gridDim.z;
+  const int kspan = ((K + gridDim.z - 1) / gridDim.z + TK - 1) / TK * TK;
   const int kbeg = blockIdx.z * kspan, kend = min(K, kbeg + kspan);
-  float acc[4][4] = {};
-  for (int k0 = kbeg; k0 < kend; k0 += TK) {
-    for (int e = threadIdx.x; e < TK * TM; e += 256) {
-      const int kk = e / TM, mm = e % TM;
+  // element x of this thread's share of a stage: consecutive threads along the stored row
+  auto a_at = [&](int x, int& kk, int& mm) {
+    const int e = tid + x * TT;
+    kk = ta ? e / TM : e % TK;
+    mm = ta ? e % TM : e / TK;
+  };
+  auto b_at = [&](int x, int& kk, int& nn) {
+    const int e = tid + x * TT;
+    kk = tb ? e % TK : e / TN;
+    nn = tb ? e / TK : e % TN;
+  };
+  float ra[TK * TM / TT], rb[TK * TN / TT];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int x = 0; x < TK * TM / TT; ++x) {
+      int kk, mm;
+      a_at(x, kk, mm);
       const int m = m0 + mm, k = k0 + kk;
-      float v = 0.f;
-      if (m < M && k < kend) v = ta ? ld(A, (long long)k * lda + m) : ld(A, (long long)m * lda + k);
-      As[kk][mm] = v;
+      ra[x] = m < M && k < kend ? (ta ? ld(A, (long long)k * lda + m) : ld(A, (long long)m * lda + k)) : 0.f;
     }
-    for (int e = threadIdx.x; e < TK * TN; e += 256) {
-      const int kk = e / TN, nn = e % TN;
+#pragma unroll
+    for (int x = 0; x < TK * TN / TT; ++x) {
+      int kk, nn;
+      b_at(x, kk, nn);
       const int n = n0 + nn, k = k0 + kk;
-      float v = 0.f;
-      if (n < N && k < kend) v = tb ? ld(B, (long long)n * ldb + k) : ld(B, (long long)k * ldb + n);
-      Bs[kk][nn] = v;
+      rb[x] = n < N && k < kend ? (tb ? ld(B, (long long)n * ldb + k) : ld(B, (long long)k * ldb + n)) : 0.f;
     }
-    __syncthreads();
+  };
+  auto stage = [&](int s) {
+#pragma unroll
+    for (int x = 0; x < TK * TM / TT; ++x) {
+      int kk, mm;
+      a_at(x, kk, mm);
+      As[s][kk][mm] = ra[x];
+    }
+#pragma unroll
+    for (int x = 0; x < TK * TN / TT; ++x) {
+      int kk, nn;
+      b_at(x, kk, nn);
+      Bs[s][kk][nn] = rb[x];
+    }
+  };
+  float acc[8][4] = {};
+  if (kbeg < kend) {
+    fetch(kbeg);
+    stage(0);
+  }
+  __syncthreads();
+  int s = 0;
+  for (int k0 = kbeg; k0 < kend; k0 += TK, s ^= 1) {
+    const bool more = k0 + TK < kend;
+    if (more) fetch(k0 + TK);
 #pragma unroll
     for (int kk = 0; kk < TK; ++kk) {
-      float a[4], b[4];
+      const float4 a0 = *reinterpret_cast<const float4*>(&As[s][kk][ty * 4]);
+      const float4 a1 = *reinterpret_cast<const float4*>(&As[s][kk][TM / 2 + ty * 4]);
+      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[s][kk][tx * 4]);
+      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, b[4] = {b0.x, b0.y, b0.z, b0.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
     }
+    if (more) stage(s ^ 1);
     __syncthreads();
   }
+  float col[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-      if (m < M && n < N) {
-        float* c = C + (long long)m * ldc + n;
-        if (gridDim.z > 1)
-          atomicAdd(c, acc[i][j]);  // C zeroed by the launcher
-        else
-          *c = beta != 0.f ? fmaf(beta, *c, acc[i][j]) : acc[i][j];
+      const int m = m0 + (i < 4 ? 0 : TM / 2) + ty * 4 + (i & 3), n = n0 + tx * 4 + j;
+      if (m >= M || n >= N) continue;
+      const long long at = (long long)m * ldc + n;
+      if (EPI == kLinear) {
+        const float z = acc[i][j] + __ldg(ep.bias + n);
+        C[at] = z;
+        ep.Y[at] = ep.silu ? silu_of(z) : z;
+      } else if (EPI == kActGrad) {
+        const float d = ep.silu ? acc[i][j] * silu_grad(__ldg(ep.Zp + at)) : acc[i][j];
+        C[at] = d;
+        col[j] += d;
+      } else if (gridDim.z > 1) {
+        atomicAdd(C + at, acc[i][j]);  // C zeroed by the launcher
+      } else {
+        C[at] = beta != 0.f ? fmaf(beta, C[at], acc[i][j]) : acc[i][j];
       }
     }
+  if (EPI == kActGrad) {
+    float* part = &As[0][0][0];  // [warp][column]: the K loop ended with a barrier
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      col[j] += __shfl_xor_sync(0xffffffffu, col[j], 16);
+      if ((tid & 16) == 0) part[(tid >> 5) * TN + tx * 4 + j] = col[j];
+    }
+    __syncthreads();
+    if (tid < TN && n0 + tid < N) {
+      float v = 0.f;
+      for (int w = 0; w < TT / 32; ++w) v += part[w * TN + tid];
+      atomicAdd(ep.db + n0 + tid, v);
+    }
+  }
 }
 
 // Z = X + b (row broadcast), Y = silu(Z) (or Y = Z); Z kept for the backward
@@ -95,7 +181,7 @@ __global__ void k_bias_act(float* Z, float* Y, const float* b, long long rows, i
   if (i >= rows * cols) return;
   const float z = Z[i] + b[i % cols];
   Z[i] = z;
-  Y[i] = silu ? z / (1.f + expf(-z)) : z;
+  Y[i] = silu ? silu_of(z) : z;
 }
 
 // dZ = dY * silu'(Z)
@@ -106,45 +192,89 @@ __global__ void k_act_grad(const float* Z, const float* dY, float* dZ, long long
     dZ[i] = dY[i];
     return;
   }
-  const float z = Z[i], s = 1.f / (1.f + expf(-z));
-  dZ[i] = dY[i] * s * (1.f + z * (1.f - s));
+  dZ[i] = dY[i] * silu_grad(Z[i]);
 }
 
-// column sums: db[c] = sum_r dZ[r, c] (row chunks of 1024, FP32 atomics; db zeroed first)
-__global__ void k_colsum(const float* dZ, float* db, long long rows, int cols) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  const long long r0 = (long long)blockIdx.y * 1024, r1 = min(rows, r0 + 1024);
+// column sums: db[c] = sum_r dZ[r, c] (32 columns x 256 rows per block, FP32 atomics; db
+// zeroed first).  One thread per column over 1024 rows: 60 us per layer of 8192 rows, 16
+// blocks; now 4
+constexpr int kSumRows = 256;
+__global__ void __launch_bounds__(256) k_colsum(const float* __restrict__ dZ, float* __restrict__ db, long long rows,
+                                                int cols) {
+  __shared__ float part[8][32];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, c = blockIdx.x * 32 + x;
+  const long long r0 = (long long)blockIdx.y * kSumRows, r1 = min(rows, r0 + kSumRows);
   float s = 0.f;
-  for (long long r = r0; r < r1; ++r) s += dZ[r * cols + c];
-  atomicAdd(db + c, s);
+  if (c < cols)
+    for (long long r = r0 + y; r < r1; r += 8) s += dZ[r * cols + c];
+  part[y][x] = s;
+  __syncthreads();
+  if (y == 0 && c < cols) {
+    for (int w = 1; w < 8; ++w) s += part[w][x];
+    atomicAdd(db + c, s);
+  }
 }
 
-__global__ void k_mse(const float* Y, const float* T, const float* mask, float* dY, double* loss, long long n,
-                      float inv_count) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  float l = 0.f;
-  if (i < n) {
+// sum of the mask (a double: exact for 0/1 masks), for k_mse
+__global__ void __launch_bounds__(256) k_mask_sum(const float* __restrict__ mask, double* __restrict__ count, long long n) {
+  __shared__ double part[8];
+  double s = 0.0;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) s += (double)mask[i];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) s += part[w];
+    atomicAdd(count, s);
+  }
+}
+
+// count non-null: 1/count is taken from the device (the mask's sum, at least 1), else inv_count.
+// One FP64 atomic per block of the grid-stride loop (one per warp of a thread per element
+// took 88 us for 8192 x 225, all on one address).
+__global__ void __launch_bounds__(256) k_mse(const float* __restrict__ Y, const float* __restrict__ T,
+                                             const float* __restrict__ mask, float* __restrict__ dY,
+                                             double* __restrict__ loss, long long n, float inv_count,
+                                             const double* __restrict__ count) {
+  __shared__ double part[8];
+  if (count) inv_count = (float)(1.0 / fmax((double)(float)*count, 1.0));
+  double l = 0.0;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
     const float d = (Y[i] - T[i]) * mask[i];
     dY[i] = 2.f * d * inv_count;
-    l = d * d * inv_count;
+    l += (double)(d * d * inv_count);
   }
   for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, (double)l);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = l;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) l += part[w];
+    atomicAdd(loss, l);
+  }
 }
 
-__global__ void k_adam(float* w, __nv_bfloat16* wb, const float* g, float* m, float* v, long long n, float lr,
-                       float b1, float b2, float eps, float c1, float c2) {
+// one Adam step of up to kAdamMax tensors (blockIdx.y)
+constexpr int kAdamMax = 8;
+struct AdamTensors {
+  float* w[kAdamMax];
+  __nv_bfloat16* wb[kAdamMax];
+  const float* g[kAdamMax];
+  float* m[kAdamMax];
+  float* v[kAdamMax];
+  long long n[kAdamMax];
+};
+__global__ void k_adam(AdamTensors t, float lr, float b1, float b2, float eps, float c1, float c2) {
+  const int y = blockIdx.y;
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float wi = w[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-  w[i] = wi;
-  if (wb) wb[i] = __float2bfloat16(wi);
+  if (i >= t.n[y]) return;
+  const float gi = t.g[y][i];
+  const float mi = b1 * t.m[y][i] + (1.f - b1) * gi;
+  const float vi = b2 * t.v[y][i] + (1.f - b2) * gi * gi;
+  t.m[y][i] = mi;
+  t.v[y][i] = vi;
+  const float wi = t.w[y][i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+  t.w[y][i] = wi;
+  if (t.wb[y]) t.wb[y][i] = __float2bfloat16(wi);
 }
 
 __global__ void k_to_bf16(const float* w, __nv_bfloat16* wb, long long n) {
@@ -162,6 +292,8 @@ int launch_fail(const char* what) {
 
 }  // namespace
 
+static const long long kFill = 304;  // blocks that fill the GPU: two per SM
+
 // C = op(A) op(B) (+ beta C): a_bf16 / b_bf16 select BF16 operands (weights)
 extern "C" int mmdg_mlp_gemm(int M, int N, int K, const void* A, int lda, int ta, int a_bf16, const void* B, int ldb,
                              int tb, int b_bf16, float* C, int ldc, float beta, void* stream) {
@@ -172,25 +304,63 @@ extern "C" int mmdg_mlp_gemm(int M, int N, int K, const void* A, int lda, int ta
   // few output tiles and a long K (weight gradients over a batch): split K over
   // enough blocks to fill the GPU, partial tiles added with atomics into a zeroed C
   const long long tiles = (long long)grid.x * grid.y;
-  if (beta == 0.f && tiles < 304 && K >= 1024) {
-    const int split = (int)std::min<long long>((K + 511) / 512, (608 + tiles - 1) / tiles);
+  if (beta == 0.f && tiles < 152 && K >= 256) {
+    const int split = (int)std::min<long long>((K + 127) / 128, (kFill + tiles - 1) / tiles);
     if (split > 1) {
       grid.z = split;
       if (cudaMemsetAsync(C, 0, sizeof(float) * (size_t)M * ldc, st) != cudaSuccess)
         return mmdg_internal_fail(MMDG_E_CUDA, "mmdg_mlp_gemm: memset");
     }
   }
+  const EpilogueArgs ep;
   if (a_bf16 && !b_bf16)
-    k_gemm<__nv_bfloat16, float><<<grid, 256, 0, st>>>(M, N, K, (const __nv_bfloat16*)A, lda, ta, (const float*)B, ldb,
-                                                        tb, C, ldc, beta);
+    k_gemm<__nv_bfloat16, float, kStore><<<grid, TT, 0, st>>>(M, N, K, (const __nv_bfloat16*)A, lda, ta,
+                                                               (const float*)B, ldb, tb, C, ldc, beta, ep);
   else if (!a_bf16 && b_bf16)
-    k_gemm<float, __nv_bfloat16><<<grid, 256, 0, st>>>(M, N, K, (const float*)A, lda, ta, (const __nv_bfloat16*)B, ldb,
-                                                        tb, C, ldc, beta);
+    k_gemm<float, __nv_bfloat16, kStore><<<grid, TT, 0, st>>>(M, N, K, (const float*)A, lda, ta,
+                                                               (const __nv_bfloat16*)B, ldb, tb, C, ldc, beta, ep);
   else if (!a_bf16 && !b_bf16)
-    k_gemm<float, float><<<grid, 256, 0, st>>>(M, N, K, (const float*)A, lda, ta, (const float*)B, ldb, tb, C, ldc, beta);
+    k_gemm<float, float, kStore><<<grid, TT, 0, st>>>(M, N, K, (const float*)A, lda, ta, (const float*)B, ldb, tb, C,
+                                                       ldc, beta, ep);
   else
     return mmdg_internal_fail(MMDG_E_ARG, "mmdg_mlp_gemm: at most one BF16 operand");
   return launch_fail("mmdg_mlp_gemm: launch");
+}
+
+// Z = X W^T + b, Y = silu(Z) or Z: X (rows x in), W BF16 (out x in)
+extern "C" int mmdg_mlp_linear(long long rows, int out, int in, const float* X, const void* W, const float* b, float* Z,
+                               float* Y, int silu, void* stream) {
+  if (!X || !W || !b || !Z || !Y || rows < 0 || rows > 0x7fffffffLL || out <= 0 || in <= 0)
+    return mmdg_internal_fail(MMDG_E_ARG, "mmdg_mlp_linear: bad argument");
+  if (!rows) return MMDG_OK;
+  EpilogueArgs ep;
+  ep.bias = b;
+  ep.Y = Y;
+  ep.silu = silu;
+  const dim3 grid((out + TN - 1) / TN, (unsigned)((rows + TM - 1) / TM));
+  k_gemm<float, __nv_bfloat16, kLinear><<<grid, TT, 0, (cudaStream_t)stream>>>(
+      (int)rows, out, in, X, in, 0, (const __nv_bfloat16*)W, in, 1, Z, out, 0.f, ep);
+  return launch_fail("mmdg_mlp_linear: launch");
+}
+
+// The step from one layer's dZ (rows x out) to the layer before: dZp = (dZ W) silu'(Zp) (or dZ W),
+// db = column sums of dZp; W BF16 (out x in), Zp, dZp (rows x in)
+extern "C" int mmdg_mlp_back(long long rows, int out, int in, const float* dZ, const void* W, const float* Zp, float* dZp,
+                             float* db, int silu, void* stream) {
+  if (!dZ || !W || !Zp || !dZp || !db || rows < 0 || rows > 0x7fffffffLL || out <= 0 || in <= 0)
+    return mmdg_internal_fail(MMDG_E_ARG, "mmdg_mlp_back: bad argument");
+  cudaStream_t st = (cudaStream_t)stream;
+  if (cudaMemsetAsync(db, 0, sizeof(float) * in, st) != cudaSuccess)
+    return mmdg_internal_fail(MMDG_E_CUDA, "mmdg_mlp_back: memset");
+  if (!rows) return MMDG_OK;
+  EpilogueArgs ep;
+  ep.Zp = Zp;
+  ep.db = db;
+  ep.silu = silu;
+  const dim3 grid((in + TN - 1) / TN, (unsigned)((rows + TM - 1) / TM));
+  k_gemm<float, __nv_bfloat16, kActGrad><<<grid, TT, 0, st>>>((int)rows, in, out, dZ, out, 0, (const __nv_bfloat16*)W,
+                                                               in, 0, dZp, in, 0.f, ep);
+  return launch_fail("mmdg_mlp_back: launch");
 }
 
 extern "C" int mmdg_mlp_bias_act(float* Z, float* Y, const float* b, long long rows, int cols, int silu, void* stream) {
@@ -213,8 +383,13 @@ extern "C" int mmdg_mlp_colsum(const float* dZ, float* db, long long rows, int c
   if (cudaMemsetAsync(db, 0, sizeof(float) * cols, st) != cudaSuccess)
     return mmdg_internal_fail(MMDG_E_CUDA, "mmdg_mlp_colsum: memset");
   if (!rows) return MMDG_OK;
-  dim3 grid(nb(cols, 128), (unsigned)((rows + 1023) / 1024));
-  k_colsum<<<grid, 128, 0, st>>>(dZ, db, rows, cols);
+  // (long batches in several launches: at most 65535 blocks along the rows)
+  const long long step = 65535LL * kSumRows;
+  for (long long r = 0; r < rows; r += step) {
+    const long long part = std::min(step, rows - r);
+    const dim3 grid(nb(cols, 32), (unsigned)((part + kSumRows - 1) / kSumRows));
+    k_colsum<<<grid, 256, 0, st>>>(dZ + r * cols, db, part, cols);
+  }
   return launch_fail("mmdg_mlp_colsum: launch");
 }
 
@@ -222,16 +397,54 @@ extern "C" int mmdg_mlp_mse(const float* Y, const float* T, const float* mask, f
                             float inv_count, void* stream) {
   if (!Y || !T || !mask || !dY || !loss || n < 0) return mmdg_internal_fail(MMDG_E_ARG, "mmdg_mlp_mse: bad argument");
   if (!n) return MMDG_OK;
-  k_mse<<<nb(n), 256, 0, (cudaStream_t)stream>>>(Y, T, mask, dY, loss, n, inv_count);
+  k_mse<<<std::min(nb(n), 608u), 256, 0, (cudaStream_t)stream>>>(Y, T, mask, dY, loss, n, inv_count, nullptr);
   return launch_fail("mmdg_mlp_mse: launch");
+}
+
+// mmdg_mlp_mse with count = max(sum of the mask, 1) taken on the device (count: a device double)
+extern "C" int mmdg_mlp_mse_masked(const float* Y, const float* T, const float* mask, float* dY, double* loss,
+                                   double* count, long long n, void* stream) {
+  if (!Y || !T || !mask || !dY || !loss || !count || n < 0)
+    return mmdg_internal_fail(MMDG_E_ARG, "mmdg_mlp_mse_masked: bad argument");
+  if (!n) return MMDG_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (cudaMemsetAsync(count, 0, sizeof(double), st) != cudaSuccess)
+    return mmdg_internal_fail(MMDG_E_CUDA, "mmdg_mlp_mse_masked: memset");
+  const unsigned blocks = std::min(nb(n), 608u);
+  k_mask_sum<<<blocks, 256, 0, st>>>(mask, count, n);
+  k_mse<<<blocks, 256, 0, st>>>(Y, T, mask, dY, loss, n, 0.f, count);
+  return launch_fail("mmdg_mlp_mse_masked: launch");
+}
+
+extern "C" int mmdg_mlp_adam_many(int count, float* const* w, void* const* w_bf16, const float* const* g,
+                                  float* const* m, float* const* v, const long long* n, float lr, float b1, float b2,
+                                  float eps, int step, void* stream) {
+  if (count < 0 || (count && (!w || !g || !m || !v || !n)) || step < 1)
+    return mmdg_internal_fail(MMDG_E_ARG, "mmdg_mlp_adam: bad argument");
+  const float c1 = 1.f / (1.f - powf(b1, (float)step)), c2 = 1.f / (1.f - powf(b2, (float)step));
+  for (int first = 0; first < count; first += kAdamMax) {
+    const int k = std::min(count - first, kAdamMax);
+    AdamTensors t;
+    long long most = 0;
+    for (int x = 0; x < k; ++x) {
+      const int y = first + x;
+      if (!w[y] || !g[y] || !m[y] || !v[y] || n[y] < 0) return mmdg_internal_fail(MMDG_E_ARG, "mmdg_mlp_adam: bad argument");
+      t.w[x] = w[y];
+      t.wb[x] = w_bf16 ? (__nv_bfloat16*)w_bf16[y] : nullptr;
+      t.g[x] = g[y];
+      t.m[x] = m[y];
+      t.v[x] = v[y];
+      t.n[x] = n[y];
+      most = std::max(most, n[y]);
+    }
+    if (most) k_adam<<<dim3(nb(most), k), 256, 0, (cudaStream_t)stream>>>(t, lr, b1, b2, eps, c1, c2);
+  }
+  return launch_fail("mmdg_mlp_adam: launch");
 }
 
 extern "C" int mmdg_mlp_adam(float* w, void* w_bf16, const float* g, float* m, float* v, long long n, float lr,
                              float b1, float b2, float eps, int step, void* stream) {
-  if (!w || !g || !m || !v || n < 0 || step < 1) return mmdg_internal_fail(MMDG_E_ARG, "mmdg_mlp_adam: bad argument");
-  const float c1 = 1.f / (1.f - powf(b1, (float)step)), c2 = 1.f / (1.f - powf(b2, (float)step));
-  k_adam<<<nb(n), 256, 0, (cudaStream_t)stream>>>(w, (__nv_bfloat16*)w_bf16, g, m, v, n, lr, b1, b2, eps, c1, c2);
-  return launch_fail("mmdg_mlp_adam: launch");
+  return mmdg_mlp_adam_many(1, &w, &w_bf16, &g, &m, &v, &n, lr, b1, b2, eps, step, stream);
 }
 
 extern "C" int mmdg_mlp_to_bf16(const float* w, void* w_bf16, long long n, void* stream) {

@@ -269,6 +269,10 @@ class DensityMLP:
             "mmdg_mlp_mse": [p, p, p, p, p, c_ll, c_f, p],
             "mmdg_mlp_adam": [p, p, p, p, p, c_ll, c_f, c_f, c_f, c_f, c_int, p],
             "mmdg_mlp_to_bf16": [p, p, c_ll, p],
+            "mmdg_mlp_linear": [c_ll, c_int, c_int, p, p, p, p, p, c_int, p],
+            "mmdg_mlp_back": [c_ll, c_int, c_int, p, p, p, p, p, c_int, p],
+            "mmdg_mlp_mse_masked": [p, p, p, p, p, p, c_ll, p],
+            "mmdg_mlp_adam_many": [c_int, p, p, p, p, p, p, c_f, c_f, c_f, c_f, c_int, p],
         }.items():
             fn = getattr(L, name)
             fn.restype = ctypes.c_int
@@ -286,11 +290,10 @@ class DensityMLP:
         for i in range(3):
             out = self.W[i].shape[0]
             Zt = torch.empty((h.shape[0], out), dtype=torch.float32, device=self.dev)
-            _native.check(L.mmdg_mlp_gemm(h.shape[0], out, h.shape[1], self._p(h), h.shape[1], 0, 0,
-                                          self._p(self.Wb[i]), h.shape[1], 1, 1, self._p(Zt), out, 0.0, st), "gemm")
             Yt = torch.empty_like(Zt)
-            _native.check(L.mmdg_mlp_bias_act(self._p(Zt), self._p(Yt), self._p(self.b[i]), h.shape[0], out,
-                                              1 if i < 2 else 0, st), "bias_act")
+            _native.check(L.mmdg_mlp_linear(h.shape[0], out, h.shape[1], self._p(h), self._p(self.Wb[i]),
+                                            self._p(self.b[i]), self._p(Zt), self._p(Yt), 1 if i < 2 else 0, st),
+                          "linear")
             acts.append((h, Zt, Yt))
             h = Yt
         return acts
@@ -302,43 +305,44 @@ class DensityMLP:
         """Gradients (dW, db) of every layer from the output gradient dY."""
         torch, L, st = self.torch, _native.lib(), _native.stream_ptr()
         grads = [None] * 3
-        d = dY
+        dZ = dY  # the last layer is linear
+        db = torch.empty(dZ.shape[1], dtype=torch.float32, device=self.dev)
+        _native.check(L.mmdg_mlp_colsum(self._p(dZ), self._p(db), dZ.shape[0], dZ.shape[1], st), "colsum")
         for i in (2, 1, 0):
-            h, Zt, _ = acts[i]
+            h = acts[i][0]
             out, inp = self.W[i].shape
-            dZ = torch.empty_like(Zt)
-            _native.check(L.mmdg_mlp_act_grad(self._p(Zt), self._p(d), self._p(dZ), dZ.numel(), 1 if i < 2 else 0, st),
-                          "act_grad")
             dW = torch.empty((out, inp), dtype=torch.float32, device=self.dev)
             _native.check(L.mmdg_mlp_gemm(out, inp, h.shape[0], self._p(dZ), out, 1, 0, self._p(h), inp, 0, 0,
                                           self._p(dW), inp, 0.0, st), "gemm dW")
-            db = torch.empty(out, dtype=torch.float32, device=self.dev)
-            _native.check(L.mmdg_mlp_colsum(self._p(dZ), self._p(db), h.shape[0], out, st), "colsum")
             grads[i] = (dW, db)
             if i > 0:
-                dh = torch.empty((h.shape[0], inp), dtype=torch.float32, device=self.dev)
-                _native.check(L.mmdg_mlp_gemm(h.shape[0], inp, out, self._p(dZ), out, 0, 0, self._p(self.Wb[i]), inp,
-                                              0, 1, self._p(dh), inp, 0.0, st), "gemm dX")
-                d = dh
+                Zp = acts[i - 1][1]
+                dZp = torch.empty_like(Zp)
+                db = torch.empty(inp, dtype=torch.float32, device=self.dev)
+                _native.check(L.mmdg_mlp_back(h.shape[0], out, inp, self._p(dZ), self._p(self.Wb[i]), self._p(Zp),
+                                              self._p(dZp), self._p(db), 1, st), "back")
+                dZ = dZp
         return grads
 
     def loss_grad(self, Y, T, M):
         torch, L, st = self.torch, _native.lib(), _native.stream_ptr()
         dY = torch.empty_like(Y)
         loss = torch.zeros(1, dtype=torch.float64, device=self.dev)
-        cnt = float(max(M.sum().item(), 1.0))
-        _native.check(L.mmdg_mlp_mse(self._p(Y), self._p(T), self._p(M), self._p(dY), self._p(loss), Y.numel(),
-                                     1.0 / cnt, st), "mse")
+        count = torch.empty(1, dtype=torch.float64, device=self.dev)
+        _native.check(L.mmdg_mlp_mse_masked(self._p(Y), self._p(T), self._p(M), self._p(dY), self._p(loss),
+                                            self._p(count), Y.numel(), st), "mse")
         return loss, dY
 
     def adam(self, grads, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         L, st = _native.lib(), _native.stream_ptr()
         self.step += 1
-        for i, (dW, db) in enumerate(grads):
-            _native.check(L.mmdg_mlp_adam(self._p(self.W[i]), self._p(self.Wb[i]), self._p(dW), self._p(self.mW[i]),
-                                          self._p(self.vW[i]), dW.numel(), lr, b1, b2, eps, self.step, st), "adam W")
-            _native.check(L.mmdg_mlp_adam(self._p(self.b[i]), None, self._p(db), self._p(self.mb[i]),
-                                          self._p(self.vb[i]), db.numel(), lr, b1, b2, eps, self.step, st), "adam b")
+        ptr = lambda ts: (ctypes.c_void_p * 6)(*[t.data_ptr() if t is not None else None for t in ts])
+        w = [*self.W, *self.b]
+        dw = [g[0] for g in grads] + [g[1] for g in grads]
+        n = (ctypes.c_longlong * 6)(*[t.numel() for t in w])
+        _native.check(L.mmdg_mlp_adam_many(6, ptr(w), ptr([*self.Wb, None, None, None]), ptr(dw),
+                                           ptr([*self.mW, *self.mb]), ptr([*self.vW, *self.vb]), n, lr, b1, b2, eps,
+                                           self.step, st), "adam")
 
     def state(self):
         out = {}
