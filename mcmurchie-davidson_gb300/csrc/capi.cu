@@ -358,7 +358,9 @@ extern "C" int mmdg_destroy(mmdg_context* h) {
 }
 
 // ------------------------------------------------------------------ pair kernel
-// One thread per shell pair: primitive-pair data (p, P) and the E' tables
+// One warp per shell pair, its lanes over the primitive pairs (one thread per shell pair was
+// a chain of up to 36 of them: 373 us for (H2O)8 6-31G**, now 141): primitive-pair data
+// (p, P) and the E' tables
 //   E'[fa fb][t u v] = c_a c_b exp(-mu |AB|^2) / p * n(fa) n(fb) * Ex_t Ey_u Ez_v
 // with the 1D Hermite expansion coefficients of cython/util.pxi:13-28 built by
 // the same recursion (base E_0^{00} = 1; the Gaussian factor is K_ab):
@@ -371,7 +373,7 @@ __device__ __forceinline__ double comp_norm(int l) { return l >= 2 ? 0.577350269
 #include "pairs.cuh"
 
 __global__ void k_build_pairs(PairBuildArgs a) {
-  const int pr = blockIdx.x * blockDim.x + threadIdx.x;
+  const int pr = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
   if (pr >= a.npair) return;
   const int sa = a.pa[pr], sb = a.pb[pr];
   const int la = a.L[sa], lb = a.L[sb];
@@ -388,7 +390,7 @@ __global__ void k_build_pairs(PairBuildArgs a) {
           nnz += (xa + xb + 1) * (ya + yb + 1) * ((la - xa - ya) + (lb - xb - yb) + 1);
   const double AB[3] = {ABx, ABy, ABz};
   const int nkeep = a.keep ? a.prc[pr] : Ka * Kb;
-  for (int k = 0; k < nkeep; ++k) {
+  for (int k = threadIdx.x & 31; k < nkeep; k += 32) {
     const int kk = a.keep ? __ldg(a.keep + a.prb[pr] + k) : k;
     const int ka = kk / Kb, kb = kk - ka * Kb;
     const double ea = a.exps[a.poff[sa] + ka], eb = a.exps[a.poff[sb] + kb];
@@ -402,30 +404,24 @@ __global__ void k_build_pairs(PairBuildArgs a) {
       a.pPf[2 * pp] = make_float4(float(p), hx, hy, hz);
       a.pPf[2 * pp + 1] = make_float4(0.f, float(Px - hx), float(Py - hy), float(Pz - hz));
     }
-    // 1D tables E[d][i][j][t], i<=2, j<=2, t<=4
+    // 1D tables E[d][i][j][t], i<=2, j<=2, t<=i+j
     double E[3][3][3][5];
     const double i2p = 0.5 * ip;
     for (int d = 0; d < 3; ++d) {
       const double XPA = -(eb * ip) * AB[d], XPB = (ea * ip) * AB[d];
-      for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j)
-          for (int t = 0; t < 5; ++t) E[d][i][j][t] = 0.0;
       E[d][0][0][0] = 1.0;
-      for (int i = 0; i < la; ++i)
-        for (int t = 0; t <= i + 1; ++t) {
-          double v = XPA * E[d][i][0][t];
-          if (t > 0) v += i2p * E[d][i][0][t - 1];
-          if (t + 1 <= i) v += (t + 1) * E[d][i][0][t + 1];
-          E[d][i + 1][0][t] = v;
-        }
-      for (int j = 0; j < lb; ++j)
-        for (int i = 0; i <= la; ++i)
-          for (int t = 0; t <= i + j + 1; ++t) {
-            double v = XPB * E[d][i][j][t];
-            if (t > 0) v += i2p * E[d][i][j][t - 1];
-            if (t + 1 <= i + j) v += (t + 1) * E[d][i][j][t + 1];
-            E[d][i][j + 1][t] = v;
+      for (int i = 0; i <= la; ++i)
+        for (int j = 0; j <= lb; ++j) {
+          if (i == 0 && j == 0) continue;
+          const int i0 = j > 0 ? i : i - 1, j0 = j > 0 ? j - 1 : 0;  // raise j if there is one, else i
+          const double X = j > 0 ? XPB : XPA;
+          for (int t = 0; t <= i + j; ++t) {
+            double v = t < i + j ? X * E[d][i0][j0][t] : 0.0;
+            if (t > 0) v += i2p * E[d][i0][j0][t - 1];
+            if (t + 1 < i + j) v += (t + 1) * E[d][i0][j0][t + 1];
+            E[d][i][j][t] = v;
           }
+        }
     }
     long long o = a.eoff[pr] + (long long)k * nnz;
     for (int xa = la; xa >= 0; --xa)
@@ -641,7 +637,7 @@ extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, i
     a.pPf = h->d_pPf.p;
     a.E64 = h->d_E64.p;
     a.E32 = h->d_E32.p;
-    k_build_pairs<<<(h->npair + 127) / 128, 128>>>(a);
+    k_build_pairs<<<(unsigned)((h->npair * 32LL + 127) / 128), 128>>>(a);
     CUDA_TRY(cudaGetLastError());
   }
   // ---- Schwarz: diagonal quartets per pair class (unsorted lists)
@@ -774,7 +770,7 @@ extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, i
       a.pPf = h->d_pPf.p;
       a.E64 = h->d_E64.p;
       a.E32 = h->d_E32.p;
-      k_build_pairs<<<(h->npair + 127) / 128, 128>>>(a);
+      k_build_pairs<<<(unsigned)((h->npair * 32LL + 127) / 128), 128>>>(a);
       CUDA_TRY(cudaGetLastError());
       CUDA_TRY(cudaDeviceSynchronize());
       npp = np2;
@@ -1513,18 +1509,31 @@ __device__ __forceinline__ void hermite_r_table(const double* boys, double p, do
 
 // One-electron integrals of the shell pairs of one pair class (la, lb) = (LA, LB),
 // cython/onee.pyx:14-192 as assembled by mmd/molecule.py:235-276.  Grid: x = pair of
-// the class list, y = nucleus of the pair's molecule (one thread per (pair, nucleus),
-// so the nuclear-attraction sums run in parallel); the y = 0 thread also writes S, T
-// and the dipole integrals; V is accumulated with atomics.  Angular momenta are
+// the class list, y = nucleus of the pair's molecule (kOneLanes threads per (pair,
+// nucleus), its primitive pairs shared among them and the sums added with shuffles; one
+// thread took the (ss) class of (H2O)8 6-31G** 324 us, 217 with eight); the y = 0 threads also
+// write S, T and the dipole integrals; V is accumulated with atomics.  Angular momenta are
 // template parameters, so every loop bound is a constant and the tables sit in
 // registers (a runtime-L version kept them in local memory: 13 ms for (H2O)16
 // 6-31G**).
+constexpr int kOneLanes = 8;
+
+// sums of n values over the threads of a group
+template <int n>
+__device__ __forceinline__ void group_sum(unsigned mask, double* v) {
+#pragma unroll
+  for (int x = 0; x < n; ++x)
+#pragma unroll
+    for (int o = 1; o < kOneLanes; o <<= 1) v[x] += __shfl_xor_sync(mask, v[x], o);
+}
+
 template <int LA, int LB>
 __global__ void __launch_bounds__(64) k_one_electron(OneEArgs a, const int* __restrict__ plist, int npair) {
   constexpr int NA = (LA + 1) * (LA + 2) / 2, NB = (LB + 1) * (LB + 2) / 2, L = LA + LB;
   constexpr int NJ = LB + 3, NT = LA + LB + 3, D = L + 1;
-  const int x0 = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x0 >= npair) return;
+  const int x0 = (blockIdx.x * blockDim.x + threadIdx.x) / kOneLanes, sub = threadIdx.x % kOneLanes;
+  if (x0 >= npair) return;  // whole groups leave together
+  const unsigned mask = ((1u << kOneLanes) - 1u) << (threadIdx.x & 31 & ~(kOneLanes - 1));
   const int pr = plist[x0];
   const int sa = a.pa[pr], sb = a.pb[pr];
   const int m = a.sh_mol[sa];
@@ -1546,88 +1555,50 @@ __global__ void __launch_bounds__(64) k_one_electron(OneEArgs a, const int* __re
   }
   const double PI = 3.141592653589793238462643383279;
   const int ka_n = a.nprim[sa], kb_n = a.nprim[sb], oa = a.poff[sa], ob = a.poff[sb];
-  for (int ka = 0; ka < ka_n; ++ka)
-    for (int kb = 0; kb < kb_n; ++kb) {
-      const double ea = a.exps[oa + ka], eb = a.exps[ob + kb];
-      const double p = ea + eb, ip = 1.0 / p, mu = ea * eb * ip;
-      const double P[3] = {(ea * A[0] + eb * B[0]) * ip, (ea * A[1] + eb * B[1]) * ip, (ea * A[2] + eb * B[2]) * ip};
-      const double cK = a.coefs[oa + ka] * a.coefs[ob + kb] * exp(-mu * AB2);
-      // 1D E[d][i][j][t], i <= LA, j <= LB + 2 (kinetic), t <= i + j (cython/util.pxi:13-28)
-      double E[3][LA + 1][NJ][NT];
-      const double i2p = 0.5 * ip;
+  for (int kk = sub; kk < ka_n * kb_n; kk += kOneLanes) {
+    const int ka = kk / kb_n, kb = kk - ka * kb_n;
+    const double ea = a.exps[oa + ka], eb = a.exps[ob + kb];
+    const double p = ea + eb, ip = 1.0 / p, mu = ea * eb * ip;
+    if (mu * AB2 > 750.0) continue;  // exp(-mu AB^2) is exactly zero
+    const double P[3] = {(ea * A[0] + eb * B[0]) * ip, (ea * A[1] + eb * B[1]) * ip, (ea * A[2] + eb * B[2]) * ip};
+    const double cK = a.coefs[oa + ka] * a.coefs[ob + kb] * exp(-mu * AB2);
+    // 1D E[d][i][j][t], i <= LA, j <= LB + 2 (kinetic), t <= i + j (cython/util.pxi:13-28)
+    double E[3][LA + 1][NJ][NT];
+    const double i2p = 0.5 * ip;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const double XPA = P[d] - A[d], XPB = P[d] - B[d];
+    for (int d = 0; d < 3; ++d) {
+      const double XPA = P[d] - A[d], XPB = P[d] - B[d];
+#pragma unroll
+      for (int i = 0; i <= LA; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+          for (int t = 0; t < NT; ++t) E[d][i][j][t] = 0.0;
+      E[d][0][0][0] = 1.0;
+#pragma unroll
+      for (int i = 0; i < LA; ++i)
+#pragma unroll
+        for (int t = 0; t <= i + 1; ++t) {
+          double v = XPA * E[d][i][0][t];
+          if (t > 0) v += i2p * E[d][i][0][t - 1];
+          if (t + 1 <= i) v += (t + 1) * E[d][i][0][t + 1];
+          E[d][i + 1][0][t] = v;
+        }
+#pragma unroll
+      for (int j = 0; j < NJ - 1; ++j)
 #pragma unroll
         for (int i = 0; i <= LA; ++i)
 #pragma unroll
-          for (int j = 0; j < NJ; ++j)
-#pragma unroll
-            for (int t = 0; t < NT; ++t) E[d][i][j][t] = 0.0;
-        E[d][0][0][0] = 1.0;
-#pragma unroll
-        for (int i = 0; i < LA; ++i)
-#pragma unroll
-          for (int t = 0; t <= i + 1; ++t) {
-            double v = XPA * E[d][i][0][t];
-            if (t > 0) v += i2p * E[d][i][0][t - 1];
-            if (t + 1 <= i) v += (t + 1) * E[d][i][0][t + 1];
-            E[d][i + 1][0][t] = v;
+          for (int t = 0; t <= i + j + 1; ++t) {
+            double v = XPB * E[d][i][j][t];
+            if (t > 0) v += i2p * E[d][i][j][t - 1];
+            if (t + 1 <= i + j) v += (t + 1) * E[d][i][j][t + 1];
+            E[d][i][j + 1][t] = v;
           }
-#pragma unroll
-        for (int j = 0; j < NJ - 1; ++j)
-#pragma unroll
-          for (int i = 0; i <= LA; ++i)
-#pragma unroll
-            for (int t = 0; t <= i + j + 1; ++t) {
-              double v = XPB * E[d][i][j][t];
-              if (t > 0) v += i2p * E[d][i][j][t - 1];
-              if (t + 1 <= i + j) v += (t + 1) * E[d][i][j][t + 1];
-              E[d][i][j + 1][t] = v;
-            }
-      }
-      const double s3 = pow(PI * ip, 1.5) * cK;
-      if (first) {  // overlap, kinetic, dipole
-        int x = 0;
-#pragma unroll
-        for (int xa = LA; xa >= 0; --xa)
-#pragma unroll
-          for (int ya = LA - xa; ya >= 0; --ya) {
-            const int za = LA - xa - ya;
-#pragma unroll
-            for (int xb = LB; xb >= 0; --xb)
-#pragma unroll
-              for (int yb = LB - xb; yb >= 0; --yb, ++x) {
-                const int zb = LB - xb - yb;
-                const double nab = comp_norm(xa) * comp_norm(ya) * comp_norm(za) * comp_norm(xb) * comp_norm(yb) *
-                                   comp_norm(zb);
-                const double Sx = E[0][xa][xb][0], Sy = E[1][ya][yb][0], Sz = E[2][za][zb][0];
-                accS[x] += nab * s3 * Sx * Sy * Sz;
-                const int lbv[3] = {xb, yb, zb};
-                const int lav[3] = {xa, ya, za};
-                double Td[3];
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                  const int l2 = lbv[d], l1 = lav[d];
-                  double t = (2 * l2 + 1) * eb * E[d][l1][l2][0] - 2.0 * eb * eb * E[d][l1][l2 + 2][0];
-                  if (l2 >= 2) t += -0.5 * l2 * (l2 - 1) * E[d][l1][l2 - 2][0];
-                  Td[d] = t;
-                }
-                accT[x] += nab * s3 * (Td[0] * Sy * Sz + Td[1] * Sx * Sz + Td[2] * Sx * Sy);
-                const double Dx = E[0][xa][xb][1] + (P[0] - O[0]) * Sx;
-                const double Dy = E[1][ya][yb][1] + (P[1] - O[1]) * Sy;
-                const double Dz = E[2][za][zb][1] + (P[2] - O[2]) * Sz;
-                accM[0][x] += nab * s3 * Dx * Sy * Sz;
-                accM[1][x] += nab * s3 * Sx * Dy * Sz;
-                accM[2][x] += nab * s3 * Sx * Sy * Dz;
-              }
-          }
-      }
-      // nuclear attraction of this thread's nucleus
-      double R[D * D * D];
-      hermite_r_table<L>(a.boys, p, P[0] - C[0], P[1] - C[1], P[2] - C[2], R);
-      const double pre = -a.atom_Z[atom] * 2.0 * PI * ip * cK;
-      int y = 0;
+    }
+    if (first) {
+      const double s3 = PI * ip * sqrt(PI * ip) * cK;  // overlap, kinetic, dipole
+      int x = 0;
 #pragma unroll
       for (int xa = LA; xa >= 0; --xa)
 #pragma unroll
@@ -1636,22 +1607,69 @@ __global__ void __launch_bounds__(64) k_one_electron(OneEArgs a, const int* __re
 #pragma unroll
           for (int xb = LB; xb >= 0; --xb)
 #pragma unroll
-            for (int yb = LB - xb; yb >= 0; --yb, ++y) {
+            for (int yb = LB - xb; yb >= 0; --yb, ++x) {
               const int zb = LB - xb - yb;
               const double nab = comp_norm(xa) * comp_norm(ya) * comp_norm(za) * comp_norm(xb) * comp_norm(yb) *
                                  comp_norm(zb);
-              double v = 0.0;
+              const double Sx = E[0][xa][xb][0], Sy = E[1][ya][yb][0], Sz = E[2][za][zb][0];
+              accS[x] += nab * s3 * Sx * Sy * Sz;
+              const int lbv[3] = {xb, yb, zb};
+              const int lav[3] = {xa, ya, za};
+              double Td[3];
 #pragma unroll
-              for (int t = 0; t <= xa + xb; ++t)
-#pragma unroll
-                for (int u = 0; u <= ya + yb; ++u)
-#pragma unroll
-                  for (int w = 0; w <= za + zb; ++w)
-                    v += E[0][xa][xb][t] * E[1][ya][yb][u] * E[2][za][zb][w] * R[(t * D + u) * D + w];
-              accV[y] += pre * nab * v;
+              for (int d = 0; d < 3; ++d) {
+                const int l2 = lbv[d], l1 = lav[d];
+                double t = (2 * l2 + 1) * eb * E[d][l1][l2][0] - 2.0 * eb * eb * E[d][l1][l2 + 2][0];
+                if (l2 >= 2) t += -0.5 * l2 * (l2 - 1) * E[d][l1][l2 - 2][0];
+                Td[d] = t;
+              }
+              accT[x] += nab * s3 * (Td[0] * Sy * Sz + Td[1] * Sx * Sz + Td[2] * Sx * Sy);
+              const double Dx = E[0][xa][xb][1] + (P[0] - O[0]) * Sx;
+              const double Dy = E[1][ya][yb][1] + (P[1] - O[1]) * Sy;
+              const double Dz = E[2][za][zb][1] + (P[2] - O[2]) * Sz;
+              accM[0][x] += nab * s3 * Dx * Sy * Sz;
+              accM[1][x] += nab * s3 * Sx * Dy * Sz;
+              accM[2][x] += nab * s3 * Sx * Sy * Dz;
             }
         }
     }
+    // nuclear attraction of this thread's nucleus
+    double R[D * D * D];
+    hermite_r_table<L>(a.boys, p, P[0] - C[0], P[1] - C[1], P[2] - C[2], R);
+    const double pre = -a.atom_Z[atom] * 2.0 * PI * ip * cK;
+    int y = 0;
+#pragma unroll
+    for (int xa = LA; xa >= 0; --xa)
+#pragma unroll
+      for (int ya = LA - xa; ya >= 0; --ya) {
+        const int za = LA - xa - ya;
+#pragma unroll
+        for (int xb = LB; xb >= 0; --xb)
+#pragma unroll
+          for (int yb = LB - xb; yb >= 0; --yb, ++y) {
+            const int zb = LB - xb - yb;
+            const double nab = comp_norm(xa) * comp_norm(ya) * comp_norm(za) * comp_norm(xb) * comp_norm(yb) *
+                               comp_norm(zb);
+            double v = 0.0;
+#pragma unroll
+            for (int t = 0; t <= xa + xb; ++t)
+#pragma unroll
+              for (int u = 0; u <= ya + yb; ++u)
+#pragma unroll
+                for (int w = 0; w <= za + zb; ++w)
+                  v += E[0][xa][xb][t] * E[1][ya][yb][u] * E[2][za][zb][w] * R[(t * D + u) * D + w];
+            accV[y] += pre * nab * v;
+          }
+      }
+  }
+  group_sum<NA * NB>(mask, accV);
+  if (first) {
+    group_sum<NA * NB>(mask, accS);
+    group_sum<NA * NB>(mask, accT);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) group_sum<NA * NB>(mask, accM[d]);
+  }
+  if (sub != 0) return;
   // scatter (each function pair belongs to exactly one shell pair); V adds this
   // nucleus's share to the zeroed matrix
   int x = 0;
@@ -1741,7 +1759,7 @@ extern "C" int mmdg_one_electron(mmdg_context* h, int natom, const int* atom_mol
     for (int lb = 0; lb <= la; ++lb) {
       const int c = pair_class(la, lb), n = h->cls_count[c];
       if (n == 0) continue;
-      const dim3 grid((n + 63) / 64, max_atoms);
+      const dim3 grid((unsigned)(((long long)n * kOneLanes + 63) / 64), max_atoms);
       const int* pl = h->d_cls[c].p;
       switch (c) {
         case 0: k_one_electron<0, 0><<<grid, 64, 0, st>>>(a, pl, n); break;

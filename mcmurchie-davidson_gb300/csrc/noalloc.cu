@@ -327,7 +327,7 @@ extern "C" int mmdg_eri_tensor_noalloc(int nshell, const int* shell_L, const int
   pa_args.pPf = nullptr;
   pa_args.E64 = dE;
   pa_args.E32 = nullptr;
-  k_build_pairs<<<(npair + 127) / 128, 128, 0, st>>>(pa_args);
+  k_build_pairs<<<(npair * 32 + 127) / 128, 128, 0, st>>>(pa_args);
   NA_TRY(cudaGetLastError());
   // ---------------- the tensor: cleared, then every class
   NA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * (size_t)nfunc * nfunc * nfunc * nfunc, st));

@@ -18,7 +18,7 @@ struct PairBuildArgs {
 };
 
 
-// One thread per shell pair: primitive-pair data and E' tables (defined in capi.cu).
+// One warp per shell pair (lanes over its primitive pairs): primitive-pair data and E' tables (defined in capi.cu).
 __global__ void k_build_pairs(PairBuildArgs a);
 
 // Boys interpolation table on the host (defined in capi.cu), written into t64
