@@ -341,18 +341,27 @@ def gen_class_warp(la, lb, lc, ld):
     s = f"{la}{lb}{lc}{ld}"
     kab = _pair_records(la, lb)
     kcd = _pair_records(lc, ld)
-    _, nnz_ab = pair_terms(la, lb)
-    _, nnz_cd = pair_terms(lc, ld)
+    bra_terms, nnz_ab = pair_terms(la, lb)
+    ket_terms, nnz_cd = pair_terms(lc, ld)
+    # Hermite index of every E' term, by E' offset; ket terms carry the parity of
+    # tau+nu+phi in bit 15
+    hpm, hqm = hidx_map(Lp), hidx_map(Lq)
+    kbt = [hpm[h] for terms in bra_terms for h, _ in terms]
+    kkt = [hqm[h] | (sum(h) % 2) << 15 for terms in ket_terms for h, _ in terms]
     o = []
     o.append(f"static __constant__ unsigned kWB_{s}[{len(kab)}] = {{{', '.join(f'{x}u' for x in kab)}}};")
     o.append(f"static __constant__ unsigned kWK_{s}[{len(kcd)}] = {{{', '.join(f'{x}u' for x in kcd)}}};")
+    o.append(f"static __constant__ unsigned char kWBT_{s}[{len(kbt)}] = {{{', '.join(map(str, kbt))}}};")
+    o.append(f"static __constant__ unsigned short kWKT_{s}[{len(kkt)}] = {{{', '.join(map(str, kkt))}}};")
     o.append(f"template <typename Real>")
     o.append(f"struct MDW_{s} {{")
     o.append(f"  static constexpr int LA = {la}, LB = {lb}, LC = {lc}, LD = {ld}, L = {L};")
     o.append(f"  static constexpr int NAB = {len(kab)}, NCD = {len(kcd)}, NNZ_AB = {nnz_ab}, NNZ_CD = {nnz_cd};")
-    o.append(f"  static constexpr int HL = {H(L)}, HP = {H(Lp)};")
+    o.append(f"  static constexpr int HL = {H(L)}, HP = {H(Lp)}, HQ = {H(Lq)};")
     o.append(f"  static __device__ __forceinline__ unsigned bra_pair(int x) {{ return kWB_{s}[x]; }}")
     o.append(f"  static __device__ __forceinline__ unsigned ket_pair(int x) {{ return kWK_{s}[x]; }}")
+    o.append(f"  static __device__ __forceinline__ unsigned char bra_term(int x) {{ return kWBT_{s}[x]; }}")
+    o.append(f"  static __device__ __forceinline__ unsigned short ket_term(int x) {{ return kWKT_{s}[x]; }}")
     o.append(f"  static __device__ __forceinline__ short herm(int x) {{ return kWH_{L}[x]; }}")
     o.append(f"}};")
     return "\n".join(o)

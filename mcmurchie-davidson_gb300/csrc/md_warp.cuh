@@ -19,8 +19,12 @@
 // function pair (the one-thread-per-(quartet, ket pair) form recomputed it up to 36
 // times), and the shared memory holds one R table per warp rather than per thread.
 // On this GPU an FP64 warp instruction occupies the FP64 pipe for ~64 cycles of its
-// sub-partition, so the integer index arithmetic and shared-memory traffic around
-// each FMA are nearly free: what counts is FP64 instructions and their lane use.
+// sub-partition, but there are 64 issue slots for it, and the index arithmetic of three
+// Hermite triples per FMA took most of them (and all of the FP32 form's time): the indices
+// come from small tables in shared memory, filled once per block -- the recursion's
+// sources, the Hermite index of every E' term, and the sum of a bra and a ket index.
+// Sum of the eight classes, (H2O)16 6-31G**, indices computed -> from tables: 11.7 -> 9.8 ms
+// FP64, 7.5 -> 5.9 ms with FP32 below 1e-5 ((dp|pp) 3.46 -> 2.82, (dd|dd) 0.38 -> 0.30).
 // Function pairs are sorted by their number of Hermite terms (generated tables), so
 // the 32 lanes of a pass run loops of nearly equal length; the remaining padding
 // issues FMAs with a zero coefficient.
@@ -38,6 +42,19 @@ constexpr int kItem = 8;  // most list quartets per warp work item (k_fock_warp)
 __device__ __forceinline__ int herm_index(int t, int u, int v) {
   const int n = t + u + v, m = n - t;
   return n * (n + 1) * (n + 2) / 6 + m * (m + 1) / 2 + (m - u);
+}
+
+// One step of the recursion for the entry (t, u, v) (packed t | u << 5 | v << 10): the first
+// non-zero index steps down, (t-1) with X, else (u-1) with Y, else (v-1) with Z.
+//   bits 0-7 its source, 8-15 the source two down (0 if none), 16-17 the coordinate,
+//   18-21 the factor of the latter
+__device__ __forceinline__ unsigned herm_step(int tuv) {
+  const int t = tuv & 31, u = (tuv >> 5) & 31, v = tuv >> 10;
+  if (tuv == 0) return 0u;
+  const int d = t > 0 ? 0 : (u > 0 ? 1 : 2), m = d == 0 ? t : (d == 1 ? u : v);
+  const int i1 = herm_index(t - (d == 0), u - (d == 1), v - (d == 2));
+  const int i2 = m > 1 ? herm_index(t - 2 * (d == 0), u - 2 * (d == 1), v - 2 * (d == 2)) : 0;
+  return (unsigned)(i1 | i2 << 8 | d << 16 | (m - 1) << 18);
 }
 
 // packed function-pair record of the generated tables:
@@ -68,7 +85,12 @@ __global__ void __launch_bounds__(kThreads) k_fock_warp(Geometry g, FockArgs f, 
   __shared__ unsigned s_pre[kMaxKeys + 1];
   __shared__ long long s_off[kMaxKeys];
   __shared__ unsigned s_ket[NCD], s_bra[NAB];
-  __shared__ short s_herm[HL];  // packed (t | u << 5 | v << 10) of every Hermite index
+  constexpr int HQ = MD::HQ;
+  __shared__ unsigned s_rec[HL];             // recursion of every entry (herm_step)
+  __shared__ Real s_fac[8];                  // 0 .. 7 (a conversion per entry costs an FP64 slot)
+  __shared__ unsigned char s_comb[HP * HQ];  // [ket Hermite index][bra Hermite index]: index of their sum
+  __shared__ unsigned short s_kt[MD::NNZ_CD];  // Hermite index (and parity, bit 15) of every ket E' term
+  __shared__ unsigned char s_bt[MD::NNZ_AB];   // Hermite index of every bra E' term
   const int nkeys = bl.nkeys;
   if (threadIdx.x < 32) {  // exclusive prefix sum of the bucket lengths
     unsigned acc = 0;
@@ -90,7 +112,14 @@ __global__ void __launch_bounds__(kThreads) k_fock_warp(Geometry g, FockArgs f, 
   }
   for (int x = threadIdx.x; x < NCD; x += kThreads) s_ket[x] = MD::ket_pair(x);
   for (int x = threadIdx.x; x < NAB; x += kThreads) s_bra[x] = MD::bra_pair(x);
-  for (int x = threadIdx.x; x < HL; x += kThreads) s_herm[x] = MD::herm(x);
+  if (threadIdx.x < 8) s_fac[threadIdx.x] = Real((int)threadIdx.x);
+  for (int x = threadIdx.x; x < HL; x += kThreads) s_rec[x] = herm_step(MD::herm(x));
+  for (int x = threadIdx.x; x < HP * HQ; x += kThreads) {
+    const int p = MD::herm(x % HP), q = MD::herm(x / HP);
+    s_comb[x] = (unsigned char)herm_index((p & 31) + (q & 31), ((p >> 5) & 31) + ((q >> 5) & 31), (p >> 10) + (q >> 10));
+  }
+  for (int x = threadIdx.x; x < MD::NNZ_CD; x += kThreads) s_kt[x] = MD::ket_term(x);
+  for (int x = threadIdx.x; x < MD::NNZ_AB; x += kThreads) s_bt[x] = MD::bra_term(x);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   extern __shared__ double smem_d[];
@@ -212,16 +241,11 @@ __global__ void __launch_bounds__(kThreads) k_fock_warp(Geometry g, FockArgs f, 
               Real* dst = (s & 1) ? R1 : R0;
               const int hs = (s + 1) * (s + 2) * (s + 3) / 6;
               for (int x2 = lane; x2 < hs; x2 += 32) {
-                const int tuv = s_herm[x2];
-                const int t = tuv & 31, u = (tuv >> 5) & 31, v = tuv >> 10;
-                // the first non-zero index steps down: (t-1) with X, else (u-1) with Y, else (v-1) with Z
-                const int d = t > 0 ? 0 : (u > 0 ? 1 : 2);
-                const int m1 = d == 0 ? t : (d == 1 ? u : v);
+                const unsigned rec = s_rec[x2];
+                const int d = (rec >> 16) & 3;
                 const Real C = d == 0 ? X : (d == 1 ? Y : Z);
-                const int i1 = herm_index(t - (d == 0), u - (d == 1), v - (d == 2));
-                const int i2 = m1 > 1 ? herm_index(t - 2 * (d == 0), u - 2 * (d == 1), v - 2 * (d == 2)) : 0;
-                Real val = C * src[x2 == 0 ? 0 : i1];
-                val = fma(Real(m1 > 1 ? m1 - 1 : 0), src[i2], val);
+                Real val = C * src[rec & 0xff];
+                val = fma(s_fac[rec >> 18], src[(rec >> 8) & 0xff], val);
                 dst[x2] = x2 == 0 ? b[L - s] : val;
               }
               __syncwarp();
@@ -233,26 +257,18 @@ __global__ void __launch_bounds__(kThreads) k_fock_warp(Geometry g, FockArgs f, 
               const bool act = o < NCD * HP;
               const int cd = act ? o / HP : 0, h = act ? o - cd * HP : 0;
               const unsigned rec = s_ket[cd];
-              const int nt = fp_nt(rec), nu = fp_nu(rec), np = fp_np(rec);
-              const int cnt = act ? nt * nu * np : 0;
+              const int cnt = act ? fp_nt(rec) * fp_nu(rec) * fp_np(rec) : 0;
               const int maxc = __reduce_max_sync(kFull, cnt);
-              const int ht = s_herm[h];
-              const int th = ht & 31, uh = (ht >> 5) & 31, vh = ht >> 10;
-              const Real* __restrict__ ep = ek + fp_eoff(rec);
+              const int e0 = fp_eoff(rec);
+              const Real* __restrict__ ep = ek + e0;
+              const unsigned char* cb = s_comb + h;
               Real w = act ? Ws[o] : Real(0);
-              int ta = 0, nv = 0, ph = 0;
+#pragma unroll 2
               for (int k = 0; k < maxc; ++k) {
                 const bool in = k < cnt;
                 const Real ev = in ? ep[k] : Real(0);
-                const Real r = Rfin[in ? herm_index(th + ta, uh + nv, vh + ph) : 0];
-                w = fma(flip_sign(ev, (ta + nv + ph) & 1), r, w);
-                if (++ph == np) {
-                  ph = 0;
-                  if (++nv == nu) {
-                    nv = 0;
-                    ++ta;
-                  }
-                }
+                const unsigned kt = in ? s_kt[e0 + k] : 0u;
+                w = fma(flip_sign(ev, (int)(kt >> 15)), Rfin[cb[(kt & 0x7fff) * HP]], w);
               }
               if (act) Ws[o] = w;
             }
@@ -266,24 +282,17 @@ __global__ void __launch_bounds__(kThreads) k_fock_warp(Geometry g, FockArgs f, 
             const bool act = o < NAB * NCD;
             const int ab = act ? o / NCD : 0, cd = act ? o - ab * NCD : 0;
             const unsigned rec = s_bra[ab];
-            const int nt = fp_nt(rec), nu = fp_nu(rec), np = fp_np(rec);
-            const int cnt = act ? nt * nu * np : 0;
+            const int cnt = act ? fp_nt(rec) * fp_nu(rec) * fp_np(rec) : 0;
             const int maxc = __reduce_max_sync(kFull, cnt);
-            const Real* __restrict__ ep = eb + fp_eoff(rec);
+            const int e0 = fp_eoff(rec);
+            const Real* __restrict__ ep = eb + e0;
             const Real* __restrict__ wr = Ws + cd * HP;
             Real a = acc[m];
-            int ta = 0, nv = 0, ph = 0;
+#pragma unroll 2
             for (int k = 0; k < maxc; ++k) {
               const bool in = k < cnt;
               const Real ev = in ? ep[k] : Real(0);
-              a = fma(ev, wr[in ? herm_index(ta, nv, ph) : 0], a);
-              if (++ph == np) {
-                ph = 0;
-                if (++nv == nu) {
-                  nv = 0;
-                  ++ta;
-                }
-              }
+              a = fma(ev, wr[in ? s_bt[e0 + k] : 0], a);
             }
             acc[m] = a;
           }
