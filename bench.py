@@ -636,7 +636,7 @@ def chosen_form_ttc(geom, ttc_plain, iters_plain, plain_mol, thr=CHOSEN_FP32_BEL
 def fp64_roofline(class_ms, counts, builds, fp64_peak):
     """FP64-pipe roofline of the Fock build from per-class CUDA-event times and counters.
 
-    Per class: ``issued`` = FP64 FLOPs the kernel issues (flop_model.issued_flops:
+    Per class: ``issued`` = FP64 FLOPs the kernel issues (flop_model.pipe_flops:
     chunk passes, padded lanes and all), ``useful`` = the algorithm's own FLOPs (no
     recomputation or padding), ``model`` = the dense reference count; each as TFLOP/s
     and as a fraction of the measured DFMA peak.  The headline is the dominant
@@ -648,7 +648,7 @@ def fp64_roofline(class_ms, counts, builds, fp64_peak):
     for c, ms, row in zip(F.CLASSES, class_ms, counts):
         if ms <= 0:
             continue
-        fl = {"issued": F.issued_flops(c, row), "useful": F.useful_flops(c, row),
+        fl = {"issued": F.pipe_flops(c, row), "useful": F.useful_flops(c, row),
               "model": F.class_flops(c, row[2], row[0])}
         for k in tot:
             tot[k] += fl[k]
@@ -659,7 +659,7 @@ def fp64_roofline(class_ms, counts, builds, fp64_peak):
     c = F.CLASSES[dom]
     key = "%d%d%d%d" % c
     row = counts[dom]
-    issued = F.issued_flops(c, row)
+    issued = F.pipe_flops(c, row)
     t = class_ms[dom] / 1e3
     achieved = issued / t / 1e12
     kern = "k_fock_warp<MDW_%s,double>" % key if F.fock_kernel(c) == "warp" else "k_fock<MD_%s,double>" % key

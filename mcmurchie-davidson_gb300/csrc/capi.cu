@@ -360,8 +360,8 @@ extern "C" int mmdg_destroy(mmdg_context* h) {
 // ------------------------------------------------------------------ pair kernel
 // One warp per shell pair, its lanes over the primitive pairs (one thread per shell pair was
 // a chain of up to 36 of them: 373 us for (H2O)8 6-31G**, now 141): primitive-pair data
-// (p, P) and the E' tables
-//   E'[fa fb][t u v] = c_a c_b exp(-mu |AB|^2) / p * n(fa) n(fb) * Ex_t Ey_u Ez_v
+// (1/p, P) and the E' tables
+//   E'[fa fb][t u v] = c_a c_b exp(-mu |AB|^2) / p^{3/2} * n(fa) n(fb) * Ex_t Ey_u Ez_v
 // with the 1D Hermite expansion coefficients of cython/util.pxi:13-28 built by
 // the same recursion (base E_0^{00} = 1; the Gaussian factor is K_ab):
 //   E^{i+1,j}_t = E^{ij}_{t-1}/(2p) + X_PA E^{ij}_t + (t+1) E^{ij}_{t+1}
@@ -396,12 +396,12 @@ __global__ void k_build_pairs(PairBuildArgs a) {
     const double ea = a.exps[a.poff[sa] + ka], eb = a.exps[a.poff[sb] + kb];
     const double p = ea + eb, ip = 1.0 / p, mu = ea * eb * ip;
     const double Px = (ea * Ax + eb * Bx) * ip, Py = (ea * Ay + eb * By) * ip, Pz = (ea * Az + eb * Bz) * ip;
-    const double K = exp(-mu * AB2) * a.coefs[a.poff[sa] + ka] * a.coefs[a.poff[sb] + kb] * ip;
+    const double K = exp(-mu * AB2) * a.coefs[a.poff[sa] + ka] * a.coefs[a.poff[sb] + kb] * (ip * sqrt(ip));
     const long long pp = a.prb[pr] + k;
-    a.pP[pp] = make_double4_32a(p, Px, Py, Pz);
+    a.pP[pp] = make_double4_32a(ip, Px, Py, Pz);
     if (a.pPf) {
       const float hx = float(Px), hy = float(Py), hz = float(Pz);
-      a.pPf[2 * pp] = make_float4(float(p), hx, hy, hz);
+      a.pPf[2 * pp] = make_float4(float(ip), hx, hy, hz);
       a.pPf[2 * pp + 1] = make_float4(0.f, float(Px - hx), float(Py - hy), float(Pz - hz));
     }
     // 1D tables E[d][i][j][t], i<=2, j<=2, t<=i+j

@@ -20,7 +20,7 @@ For every angular class (la lb|lc ld) with la>=lb, lc>=ld, (la,lb)>=(lc,ld)
 This is the algorithm of the reference's ``electron_repulsion`` + ``ERI``
 (cython/twoe.pyx:36-94) with its loops reordered: the E products are formed once
 per primitive pair (E' tables, built by the pair kernel with the contraction
-coefficients, normalisation and 1/p folded in), the R recursion (cython/util.pxi:33-50)
+coefficients, normalisation and p^-3/2 folded in), the R recursion (cython/util.pxi:33-50)
 is evaluated once per primitive quartet for all (t,u,v) instead of recursively per
 term, and the six-fold Hermite sum is factorised into a ket transform (per
 primitive quartet) and a bra transform (per bra primitive).
@@ -31,7 +31,7 @@ per-thread slice of shared memory.  The chunk size per class is a tunable.
 
 The E' table layout (shared with pairs.cu): for fa in comps(la), fb in comps(lb)
 (row-major), for t <= xa+xb, u <= ya+yb, v <= za+zb (t outermost):
-    E'[fa fb][t u v] = c K_ab / p * norm_a norm_b * Ex_t Ey_u Ez_v.
+    E'[fa fb][t u v] = c K_ab / p^(3/2) * norm_a norm_b * Ex_t Ey_u Ez_v.
 """
 from __future__ import annotations
 

@@ -12,7 +12,7 @@
 //     d/dA = (a/p) d/dP + d/d(A-B),      d/dB = (b/p) d/dP - d/d(A-B),
 // and d/dP raises a Hermite index by one.  So per primitive pair the kernels need the
 // coefficients E' of the ERI code (cython/util.pxi:13-28, contraction, normalisation and
-// 1/p folded in) and their three derivatives with respect to A - B, tabulated once per
+// p^{-3/2} folded in) and their three derivatives with respect to A - B, tabulated once per
 // gradient (k_grad_pairs); centre-differentiated functions (2a G_{i+1} - i G_{i-1},
 // cython/grad.pyx:101-108) are needed for the kinetic energy only.
 #include <cuda_runtime.h>
@@ -55,7 +55,7 @@ __host__ __device__ constexpr int comp_y(int L, int c) {
 }
 
 // ------------------------------------------------------------------ primitive-pair tables
-// One thread per primitive pair: (p, P), a/p, the coefficients E' in the layout of the ERI
+// One thread per primitive pair: (1/p, P), a/p, the coefficients E' in the layout of the ERI
 // code (component pairs row-major, then t, u, v) and, behind 3 x the same offset, their
 // derivatives with respect to A - B along x, y, z.  With X_PA = -(b/p) (A-B)_x and X_PB =
 // (a/p) (A-B)_x the recursion E^{i+1,j}_t = E^{ij}_{t-1}/(2p) + X_PA E^{ij}_t + (t+1)
@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(64) k_grad_pairs(GradArgs a) {
     AB2 += AB[d] * AB[d];
     P[d] = (ea * A + eb * B) * ip;
   }
-  const double K = exp(-mu * AB2) * a.coefs[a.poff[sa] + ka] * a.coefs[a.poff[sb] + kb] * ip;
-  a.pP[pp] = make_double4_32a(p, P[0], P[1], P[2]);
+  const double K = exp(-mu * AB2) * a.coefs[a.poff[sa] + ka] * a.coefs[a.poff[sb] + kb] * (ip * sqrt(ip));
+  a.pP[pp] = make_double4_32a(ip, P[0], P[1], P[2]);
   a.frac[pp] = ea * ip;
   double E[3][3][3][5], D[3][3][3][5];
   for (int d = 0; d < 3; ++d) {
@@ -231,7 +231,7 @@ struct GradTab {
   }
 };
 
-// R^(n)_000, n = 0..M, with the 1/sqrt(p+q) of the ERI code.  M = 9 ((dd|dd)) is one order
+// R^(n)_000, n = 0..M, with the sqrt(alpha) of the ERI code.  M = 9 ((dd|dd)) is one order
 // past the Boys table: its series and downward recursion below T = 48, else upward
 // recursion off F_0
 template <int M>
@@ -246,7 +246,7 @@ __device__ __forceinline__ void hermite_r0_grad(const Geometry& g, const double4
     X = a.y - b.y;
     Y = a.z - b.z;
     Z = a.w - b.w;
-    const double r = rsqrt_dd(a.x + b.x), alpha = a.x * b.x * (r * r);
+    const double r = rsqrt_dd(a.x + b.x), alpha = r * r;
     const double T = alpha * fma(X, X, fma(Y, Y, Z * Z)), e = exp(-T);
     double F[M + 1];
     if (T < 48.0) {
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kGradThreads) k_grad_nuclei(GradArgs a, Geomet
   const int count = a.prc[pr], first = a.prb[pr];
   double* grad = a.grad + (long long)(blockIdx.x % kGradCopies) * 3 * a.natom;
   double gA[3] = {0, 0, 0}, gP[3] = {0, 0, 0};
-  // attraction -Z (2 pi / p) K E ... from E' = sqrt(2 pi^{5/2}) K / p E ...; both orders of two
+  // attraction -Z (2 pi / p) K E ... from E' = sqrt(2 pi^{5/2}) K p^{-3/2} E ...; both orders of two
   // different shells, and 2 P_ij
   const double pre = -2.0 * kPi / kSqrtTwoPi52 * 2.0 * (sa == sb ? 1.0 : 2.0);
   for (int it = lane; it < count * a.natom; it += 32) {
@@ -556,14 +556,15 @@ __global__ void __launch_bounds__(kGradThreads) k_grad_nuclei(GradArgs a, Geomet
       }
     }
     const double4_32a pp = g.pP[first + k];
+    const double pe = 1.0 / pp.x;  // p
     const double X = pp.y - a.xyz[3 * c], Y = pp.z - a.xyz[3 * c + 1], Z = pp.w - a.xyz[3 * c + 2];
     double F[M + 1], R[hcount(M)];
-    boys_eval<M>(g.boys64, pp.x * fma(X, X, fma(Y, Y, Z * Z)), F);
-    double f = pre * a.Z[c];
+    boys_eval<M>(g.boys64, pe * fma(X, X, fma(Y, Y, Z * Z)), F);
+    double f = pre * sqrt(pe) * a.Z[c];
 #pragma unroll
     for (int m = 0; m <= M; ++m) {
       F[m] *= f;
-      f *= -2.0 * pp.x;
+      f *= -2.0 * pe;
     }
     R[0] = F[M];
 #pragma unroll

@@ -19,7 +19,7 @@ struct GradArgs {
   int nprimpair;
   const int *prb, *prc, *pair_nnz, *pp_pair, *pp_index;
   const long long* eoff;
-  double4_32a* pP;  // (p, P)
+  double4_32a* pP;  // (1/p, P)
   double* frac;     // a / p
   double* E64;      // E' tables
   double* ER;       // d E' / d(A-B), at 3 x the offset of E', x, y and z after one another

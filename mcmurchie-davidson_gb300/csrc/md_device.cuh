@@ -33,7 +33,8 @@ constexpr int kBoysDfRow = 16;
 constexpr double kTwoPi52 = 34.986836655249725;  // 2 pi^{5/2}
 // sqrt(2 pi^{5/2}): folded into every E' coefficient by the pair kernel, so the
 // product of a bra and a ket coefficient carries the 2 pi^{5/2} of the primitive ERI
-// (cython/twoe.pyx:93) and the quartet code multiplies by 1/sqrt(p+q) only
+// (cython/twoe.pyx:93); with p^{-3/2} beside it the quartet code multiplies by
+// sqrt(alpha) only
 constexpr double kSqrtTwoPi52 = 5.914967172795613;
 constexpr double kHalfSqrtPi = 0.88622692545275801;
 
@@ -71,21 +72,74 @@ __device__ __forceinline__ float f32_of_double_tz(double x) {
                  : __int_as_float((hi & 0x80000000) | (fe << 23) | ((hi & 0xfffff) << 3) | (int)(lo >> 29));
 }
 
+// an unevaluated sum of two floats (see the double-float arithmetic below)
+struct DF {
+  float hi, lo;
+};
+
+// a double as a float pair on the integer pipe: hi = the top 24 significant bits,
+// lo = the next 29 rounded to 24 (|x| below 2^-74: lo = 0; below 2^-126: 0)
+__device__ __forceinline__ DF df_of_double(double x) {
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  const int e = (hi >> 20) & 0x7ff;
+  const int sign = hi & 0x80000000;
+  if (e < 1023 - 126) return {0.0f, 0.0f};
+  const float h = __int_as_float(sign | ((e - (1023 - 127)) << 23) | ((hi & 0xfffff) << 3) | (int)(lo >> 29));
+  float l = 0.0f;
+  if (e >= 1023 - 74) {
+    const float scale = __int_as_float((e - 1075 + 127) << 23);  // 2^(e - 1075)
+    l = __int2float_rn((int)(lo & 0x1fffffffu)) * scale;
+    l = sign ? -l : l;
+  }
+  return {h, l};
+}
+
+// (2^52 + frac) 2^(exp - 52) from its fraction in units of 2^(exp - 52), which may have left
+// [0, 2^52) by less than a binade: below, the unit is half as long; above, twice
+__device__ __forceinline__ double f64_assemble(int exp, long long frac) {
+  constexpr long long kOne = 1LL << 52;
+  if (frac < 0) frac <<= 1;
+  else if (frac >= kOne) frac = kOne + ((frac - kOne + 1) >> 1);
+  return __longlong_as_double(((long long)(exp + 1023) << 52) + frac);
+}
+
 // 1/sqrt(x) for a positive double whose magnitude is within the normal float range:
 // the single-precision estimate y0 = rsqrtf(x) (special-function unit; x and y0
 // moved between formats on the integer pipe) and one third-order step of the
 // Newton/Householder iteration for the inverse square root,
 //     e = 1 - x y0^2,   y = y0 (1 + e/2 + 3 e^2/8) = y0 + (y0/2) (e + (3e/4) e),
 // whose error is 5/16 e^3 + O(e^4); |e| < 2^-20 leaves it far below double rounding.
-// The factor 3e/4 only scales a term below 2^-40 of the result, so it is taken from
-// the FP32 pipe (24 bits), and y0/2 is exact in FP32: four FP64 instructions (a
-// product and three FMAs), the same rounding as the all-FP64 step.
+// One FP64 instruction: e, of an exact y0^2 squared as a 24-bit integer.  The correction,
+// below 2^-20 of y0, is formed as a float pair (e split exactly, y0 e exact by an FMA, the
+// e^2 term in FP32) and added to y0's fraction in integer arithmetic, rounded once.  An
+// FP64 instruction holds its pipe for 64 issue slots, these steps take some 50.  The same
+// step in four FP64 instructions: (ss|ss) 1.69 against 1.44 ms, (ps|ss) 3.63 against 3.34 on
+// (H2O)16 6-31G**, 48 clusters 6-31G 22.6 against 21.1 ms per build.
 __device__ __forceinline__ double rsqrt_dd(double x) {
-  const float y0f = rsqrtf(f32_of_nonneg(x));
-  const double y0 = f64_of_positive(y0f);
-  const double e = fma(-x, y0 * y0, 1.0);  // y0 has 24 significant bits: y0^2 is exact
-  const double b = fma(f64_of_float(0.75f * f32_of_double_tz(e)), e, e);  // e + 3e^2/4
-  return fma(f64_of_positive(0.5f * y0f), b, y0);
+  const float y0 = rsqrtf(f32_of_nonneg(x));
+  const int yb = __float_as_int(y0), exp = (yb >> 23) - 127;
+  const unsigned m = (yb & 0x7fffff) | 0x800000;
+  const unsigned long long sq = (unsigned long long)m * m;  // 2^46 <= sq < 2^48
+  const int top = (int)(sq >> 47);
+  const double y02 = __longlong_as_double(((long long)(2 * exp + top + 1022) << 52) + (long long)(sq << (6 - top)));
+  const double e = fma(-x, y02, 1.0);
+  const DF ed = df_of_double(e);
+  const float p = ed.hi * y0;
+  const float lo = fmaf(y0, fmaf(0.75f * ed.hi, ed.hi, ed.lo), fmaf(ed.hi, y0, -p));
+  const float unit = __int_as_float((51 - exp + 127) << 23);  // half the correction in units of 2^(exp - 52)
+  const float h = p * unit;                                   // below 2^31.4: taken off in steps of two
+  const int h2 = __float2int_rn(0.5f * h);
+  const int rest = __float2int_rn(fmaf(lo, unit, fmaf(-2.0f, __int2float_rn(h2), h)));
+  return f64_assemble(exp, ((long long)(yb & 0x7fffff) << 29) + 2LL * h2 + rest);
+}
+
+// hi + lo as a double, for a normal hi > 0 of at least 2^-75 and |lo| <= ulp(hi)/2, rounded to
+// nearest in integer arithmetic
+__device__ __forceinline__ double f64_of_pair(DF a) {
+  const int b = __float_as_int(a.hi), exp = (b >> 23) - 127;
+  const int lo = __float2int_rn(a.lo * __int_as_float((52 - exp + 127) << 23));
+  return f64_assemble(exp, ((long long)(b & 0x7fffff) << 29) + lo);
 }
 
 // (-1)^s x by an integer XOR of the sign bit.  A select between x and -x compiles to
@@ -102,8 +156,8 @@ __device__ __forceinline__ float flip_sign(float x, int s) {
 // geometry shared by every kernel
 struct Geometry {
   // primitive pairs
-  const double4_32a* __restrict__ pP;   // (p, Px, Py, Pz) per primitive pair
-  const float4* __restrict__ pPf;   // FP32: (p, Px, Py, Pz) rounded, then (0, Px, Py, Pz) remainders: 2 per pair
+  const double4_32a* __restrict__ pP;   // (1/p, Px, Py, Pz) per primitive pair
+  const float4* __restrict__ pPf;   // FP32: (1/p, Px, Py, Pz) rounded, then (0, Px, Py, Pz) remainders: 2 per pair
   const double* __restrict__ E64;   // E' tables, FP64
   const float* __restrict__ E32;    // E' tables, FP32
   // shell pairs
@@ -237,9 +291,6 @@ __device__ __forceinline__ void boys_eval(const float* __restrict__ tab, float T
 // Knuth's two-sum, with the FMA giving exact products: a value is hi + lo with
 // |lo| <= ulp(hi)/2, about 48 significant bits.  Used where a result needs ~1e-14
 // relative accuracy and the FP64 pipe (1/61 of the FP32 rate here) is the bottleneck.
-struct DF {
-  float hi, lo;
-};
 __device__ __forceinline__ DF df_two_sum(float a, float b) {
   const float s = a + b;
   const float bb = s - a;
@@ -257,24 +308,6 @@ __device__ __forceinline__ DF df_fma(DF a, DF y, DF c) {
   e = fmaf(a.lo, y.hi, e);
   DF s = df_two_sum(p, c.hi);
   return df_fast_two_sum(s.hi, s.lo + (e + c.lo));
-}
-
-// a double as a float pair on the integer pipe: hi = the top 24 significant bits,
-// lo = the next 29 rounded to 24 (|x| below 2^-74: lo = 0; below 2^-126: 0)
-__device__ __forceinline__ DF df_of_double(double x) {
-  const int hi = __double2hiint(x);
-  const unsigned lo = (unsigned)__double2loint(x);
-  const int e = (hi >> 20) & 0x7ff;
-  const int sign = hi & 0x80000000;
-  if (e < 1023 - 126) return {0.0f, 0.0f};
-  const float h = __int_as_float(sign | ((e - (1023 - 127)) << 23) | ((hi & 0xfffff) << 3) | (int)(lo >> 29));
-  float l = 0.0f;
-  if (e >= 1023 - 74) {
-    const float scale = __int_as_float((e - 1075 + 127) << 23);  // 2^(e - 1075)
-    l = __int2float_rn((int)(lo & 0x1fffffffu)) * scale;
-    l = sign ? -l : l;
-  }
-  return {h, l};
 }
 
 // sum_{n >= 1} c_n y^(n-1) over one table row (n up to 6, or 7 for an exp row), as a
@@ -300,12 +333,12 @@ template <int DEG>
 __device__ __forceinline__ double df_row(const float* __restrict__ row, const double* __restrict__ row64, double y,
                                          DF ydf) {
   const DF t = df_row_tail<DEG>(row, ydf);
-  return fma(y, f64_of_float(t.hi) + f64_of_float(t.lo), __ldg(row64));
+  return fma(y, f64_of_pair(t), __ldg(row64));  // t = c_1 + ... > 0
 }
 
 // Fn[0..L] for T < 48 - 1/32 from boys_eval's table with the Taylor rows evaluated
-// mostly on the FP32 pipe: per row one FP64 add and one FP64 FMA (plus y = T_k - T
-// once) instead of six FMAs; for L > 1 the exp row likewise, the downward recursion
+// mostly on the FP32 and integer pipes: per row one FP64 FMA (plus y = T_k - T once)
+// instead of six; for L > 1 the exp row likewise, the downward recursion
 // stays FP64.  Relative error of a row 2.2e-16 against its FP64 Horner evaluation
 // (emulated over T < 48, L <= 4 and the exp rows).  T at or past the table takes
 // boys_eval's asymptotic branch, and so does every T when the geometry carries no
@@ -365,17 +398,19 @@ struct Ctx<double> {
   __device__ __forceinline__ void hermite_r0(int i, int j, double* Rn, double& X, double& Y, double& Z) const {
     hermite_r0_pp<L>(g->pP[i], g->pP[j], Rn, X, Y, Z);
   }
-  // R^(n)_000 = (p+q)^{-1/2} (-2 alpha)^n F_n(T), n = 0..L, T = alpha |PQ|^2, alpha =
-  // pq/(p+q), and PQ = (X, Y, Z).  For L <= 4 the branch is taken before any FP64
-  // work that only one side needs, on an FP32 estimate of T (FP32 and integer pipes):
-  //   near (T < 48 - 1/32): 1/sqrt(p+q), alpha, T, the tabulated Boys function;
+  // R^(n)_000 = sqrt(alpha) (-2 alpha)^n F_n(T), n = 0..L, T = alpha |PQ|^2, alpha =
+  // pq/(p+q) = 1/(1/p + 1/q), and PQ = (X, Y, Z): the primitive ERI's 1/(pq sqrt(p+q)) is
+  // sqrt(alpha) (pq)^{-3/2}, whose p^{-3/2} is in the E' coefficients, so a primitive pair
+  // brings 1/p and a quartet needs no product or sum of p and q but 1/alpha.  For L <= 4
+  // the branch is taken before any FP64 work that only one side needs, on an FP32
+  // estimate of T (FP32 and integer pipes):
+  //   near (T < 48 - 1/32): sqrt(alpha), T, the tabulated Boys function;
   //   far: the asymptotic F_n = (2n-1)!! sqrt(pi) / (2^{n+1} T^{n+1/2}) (the e^{-T}
   //   terms are below 5e-15 relative for n <= 4) turns R^(n) into the point-charge
-  //   form R^(0) = sqrt(pi)/2 / (sqrt(pq) |PQ|), R^(n) = -(2n-1) R^(n-1) / |PQ|^2,
-  //   which needs 1/sqrt(pq |PQ|^2) and no Boys function or alpha at all.
+  //   form R^(0) = sqrt(pi)/2 / |PQ|, R^(n) = -(2n-1) R^(n-1) / |PQ|^2.
   // Both sides are one product chain, R^(n) = rr M^n B_n, with
-  //   near: rr = 1/sqrt(p+q),      M = -2 pq rr^2 = -2 alpha, B_n = F_n(T);
-  //   far:  rr = 1/sqrt(pq |PQ|^2), M = -pq rr^2 = -1/|PQ|^2,  B_n = (2n-1)!! sqrt(pi)/2,
+  //   near: rr = 1/sqrt(1/p + 1/q) = sqrt(alpha), M = -2 rr^2 = -2 alpha, B_n = F_n(T);
+  //   far:  rr = 1/|PQ|,                          M = -rr^2,              B_n = (2n-1)!! sqrt(pi)/2,
   // so a warp whose lanes straddle T = 48 (most warps of the s and p classes: far
   // primitive quartets outnumber near ones about 4 to 1 in water clusters) issues the
   // reciprocal square root and the chain once, and only T and the Boys rows on the
@@ -390,11 +425,11 @@ struct Ctx<double> {
     Z = a.w - b.w;
     const double r2 = fma(X, X, fma(Y, Y, Z * Z));
     if constexpr (L <= 4) {
-      const double pq = a.x * b.x, s = a.x + b.x, pqr2 = pq * r2;
-      const float Tf = __fdividef(f32_of_nonneg(pqr2), f32_of_nonneg(s));
+      const double ia = a.x + b.x;  // 1/alpha
+      const float Tf = __fdividef(f32_of_nonneg(r2), f32_of_nonneg(ia));
       const bool far = Tf >= float(kBoysTaylorMax);
-      const double rr = rsqrt_dd(far ? pqr2 : s);
-      const double pqrr2 = pq * (rr * rr);  // near: alpha; far: 1/|PQ|^2
+      const double rr = rsqrt_dd(far ? r2 : ia);
+      const double rr2 = rr * rr;  // near: alpha; far: 1/|PQ|^2
       double B[L + 1];
       if (far) {
         ++nasym;
@@ -405,13 +440,13 @@ struct Ctx<double> {
           f *= double(2 * n + 1);  // compile-time constants
         }
       } else {
-        boys_eval_df<L>(g->boysdf, g->boys64, pqrr2 * r2, B);
+        boys_eval_df<L>(g->boysdf, g->boys64, rr2 * r2, B);
       }
       double c = rr;  // 2 pi^{5/2} is folded into the E' coefficients
       Rn[0] = c * B[0];
       if (L > 0) {
-        const unsigned hm = ((unsigned)__double2hiint(pqrr2) ^ 0x80000000u) + (far ? 0u : 0x00100000u);
-        const double M = __hiloint2double((int)hm, __double2loint(pqrr2));
+        const unsigned hm = ((unsigned)__double2hiint(rr2) ^ 0x80000000u) + (far ? 0u : 0x00100000u);
+        const double M = __hiloint2double((int)hm, __double2loint(rr2));
 #pragma unroll
         for (int n = 1; n <= L; ++n) {
           c *= M;
@@ -420,13 +455,13 @@ struct Ctx<double> {
       }
       return;
     }
-    const double rsum = rsqrt_dd(a.x + b.x);
-    const double alpha = a.x * b.x * (rsum * rsum);
+    const double ra = rsqrt_dd(a.x + b.x);  // sqrt(alpha)
+    const double alpha = ra * ra;
     double F[L + 1];
     const double T = alpha * r2;
     nasym += f32_of_nonneg(T) >= float(kBoysTaylorMax) ? 1u : 0u;
     boys_eval<L>(g->boys64, T, F);
-    double c = rsum;  // 2 pi^{5/2} is folded into the E' coefficients
+    double c = ra;  // 2 pi^{5/2} is folded into the E' coefficients
     const double m2a = -2.0 * alpha;
 #pragma unroll
     for (int n = 0; n <= L; ++n) {
@@ -457,7 +492,7 @@ struct Ctx<float> {
     return g->E32 + ebra + (long long)(i - bra_begin) * nnz_ab;
   }
   struct PP {
-    float4 hi;  // (p, P) rounded to FP32
+    float4 hi;  // (1/p, P) rounded to FP32
     float4 lo;  // (0, P - hi): P as an unevaluated float pair
   };
   __device__ __forceinline__ PP pp(int k) const { return PP{g->pPf[2 * k], g->pPf[2 * k + 1]}; }
@@ -474,14 +509,13 @@ struct Ctx<float> {
     Y = (a.hi.z - b.hi.z) + (a.lo.z - b.lo.z);
     Z = (a.hi.w - b.hi.w) + (a.lo.w - b.lo.w);
     const float r2 = fmaf(X, X, fmaf(Y, Y, Z * Z));
-    const float pa = a.hi.x, pb = b.hi.x;
-    const float rsum = rsqrtf(pa + pb);
-    const float alpha = pa * pb * (rsum * rsum);
+    const float ra = rsqrtf(a.hi.x + b.hi.x);  // sqrt(alpha)
+    const float alpha = ra * ra;
     float F[L + 1];
     const float T = alpha * r2;
     nasym += T >= float(kBoysTaylorMax) ? 1u : 0u;
     boys_eval<L>(g->boys32, T, F);
-    float c = rsum;  // 2 pi^{5/2} is folded into the E' coefficients
+    float c = ra;  // 2 pi^{5/2} is folded into the E' coefficients
     const float m2a = -2.0f * alpha;
 #pragma unroll
     for (int n = 0; n <= L; ++n) {

@@ -91,9 +91,13 @@ def build_flops(counts, kind: str = "model") -> float:
 
 
 # ------------------------------------------------------------------ issued / useful FP64 FLOPs
-# What the Fock kernels really issue, counted from the structure of the generated
+# The FP64 arithmetic of the Fock kernels, counted from the structure of the generated
 # code (csrc/gen_md.py, csrc/md_device.cuh, csrc/md_warp.cuh), lane by lane, with an
-# FMA as 2 FLOPs and a multiply or add as 1 -- the quantity that ncu's
+# FMA as 2 FLOPs and a multiply or add as 1.  ``issued_flops`` counts every operation of
+# the step's FP64 form (``r0_flops``: products and sum of p and q, the reciprocal square
+# root in four FP64 instructions, one conversion sum per Boys row); ``pipe_flops`` what
+# the FP64 pipe is given of it, with 1/alpha from tabulated 1/p and the square root's and
+# the rows' last steps done exactly on the integer pipe -- the quantity that ncu's
 # smsp__sass_thread_inst_executed_op_{dfma,dmul,dadd}_pred_on counters measure as
 # 2 DFMA + DMUL + DADD.  Not counted: the FP64 instructions inside CUDA's exp
 # (library code, called only by the asymptotic Boys branch of L >= 5), conversions
@@ -165,6 +169,23 @@ def r0_flops(L: int, asymptotic: bool) -> int:
     return 3 + 5 + 1 + RSQRT_FLOPS + 3 + 1 + boys_flops(L, asymptotic) + pref
 
 
+def r0_pipe_flops(L: int, asymptotic: bool) -> int:
+    """What of r0_flops reaches the FP64 pipe: P - Q (3), |PQ|^2 (5), 1/alpha = 1/p + 1/q (1),
+    the e of rsqrt_dd (2), rr^2 (1; for L = 0 only near), near: T (1), y = T_k - T (1), the
+    last FMA of each Boys row (2) and the downward recursion; the product chain.  L >= 5:
+    the same start, alpha, T, boys_eval (its square root, if any, one FMA) and the
+    prefactor powers."""
+    start = 3 + 5 + 1 + 2
+    saved = (RSQRT_FLOPS - 2) if asymptotic else 0
+    if L > 4:
+        return start + 1 + 1 + boys_flops(L, asymptotic) - saved + 1 + (2 * L + 1)
+    chain = 1 + 2 * L
+    if asymptotic:
+        return start + (0 if L == 0 else 1) + chain
+    rows = 1 if L == 0 else 2
+    return start + 1 + 1 + boys_df_flops(L) - rows + chain
+
+
 @lru_cache(maxsize=None)
 def recursion_flops(L: int) -> int:
     """The in-place Hermite Coulomb recursion of the per-thread code: X R1 (1 FLOP) when
@@ -228,6 +249,16 @@ def issued_flops(cls, row) -> float:
         return r0 + npq * (rlev + ket) + nbp * bra + 6.0 * nfq
     nch, ket, bra = _thread_config(tuple(cls))
     return nch * (r0 + npq * recursion_flops(L)) + npq * ket + nbp * bra + 6.0 * nfq
+
+
+def pipe_flops(cls, row) -> float:
+    """The FLOPs of ``issued_flops`` that run on the FP64 pipe."""
+    npq, nas = float(row[2]), float(row[4]) if len(row) > 4 else 0.0
+    L = sum(cls)
+    off = (npq - nas) * (r0_flops(L, False) - r0_pipe_flops(L, False)) + \
+        nas * (r0_flops(L, True) - r0_pipe_flops(L, True))
+    passes = 1 if fock_kernel(cls) == "warp" else _thread_config(tuple(cls))[0]
+    return issued_flops(cls, row) - passes * off
 
 
 def useful_flops(cls, row) -> float:
