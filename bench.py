@@ -815,9 +815,9 @@ def gpu_arm(args):
                    "quartets_per_s_1core": cb["quartets_per_s_1core"], "anchor": cb.get("anchor")}
         except Exception as e:  # the baseline is reported, never required
             cpu = {"value": None, "error": str(e)[:300]}
-    # our kernels per Fock build: k_prep_density, k_shell_dmax, one k_screen per class,
-    # one k_fock per class and precision, and k_fock_update of the SCF step
-    launches_per_build = 3 + len(flop_model.CLASSES) * (3 if fp32 > 0 else 2)
+    # our kernels per Fock build: k_shell_dmax, k_screen, one k_fock per class and
+    # precision, and k_fock_update of the SCF step
+    launches_per_build = 3 + len(flop_model.CLASSES) * (2 if fp32 > 0 else 1)
     batched = mixed = combined = None
     if rank == 0 and not args.no_batch:
         try:
@@ -853,7 +853,7 @@ def gpu_arm(args):
         "roofline": roofline, "cpu_baseline": cpu, "clocks": clk,
         "gpu_launches": launches_per_build * builds, "wall_s": wall,
         "step_breakdown_ms": {"step": 1e3 * t_dev / builds, "fock_class_kernels_one_stream": build_ms,
-                              "note": "the timed steps run the class kernels on 4 concurrent streams; the "
+                              "note": "the timed steps run the class kernels on 8 concurrent streams; the "
                                       "per-class profile replays the same densities on one stream"},
         "batched": batched, "mixed_precision": mixed, "combined_form": combined, "consumers": consumers,
         "class_ms_per_build": {"%d%d%d%d" % c: float(x) / builds for c, x in zip(flop_model.CLASSES, class_ms)},

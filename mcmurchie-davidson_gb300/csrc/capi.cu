@@ -252,8 +252,19 @@ struct mmdg_context {
   int part = 0, nparts = 1;
   // screening / Fock scratch
   DevBuf<double> d_screen, d_sq;
-  DevBuf<float> d_sqf, d_dPf, d_Dsh;
-  DevBuf<unsigned long long> d_counters;
+  DevBuf<float> d_sqf, d_Dsh;
+  // what a build starts from zero, in one piece: the counters [kCounters * MMDG_NCLASS], the work
+  // counters of the FP64 and FP32 class launches [2 * MMDG_NCLASS], the largest |dP| of every
+  // molecule [nmol], the FP64 and FP32 bucket lengths [2 * total_keys]
+  DevBuf<unsigned long long> d_zero;
+  size_t dmax_words = 0;
+  unsigned long long* counters() const { return d_zero.p; }
+  unsigned long long* work() const { return d_zero.p + kCounters * MMDG_NCLASS; }
+  float* dmax() const { return reinterpret_cast<float*>(work() + 2 * MMDG_NCLASS); }
+  unsigned* lengths() const { return reinterpret_cast<unsigned*>(dmax() + 2 * dmax_words); }
+  DevBuf<float> d_qtile[kNumPairClasses];  // largest Q of every tile of the class lists
+  DevBuf<ScreenClass> d_screens;           // the screening pass's classes
+  int nscreen = 0, screen_blocks = 0;
   // quartet lists of the Fock build (allocated on first use): per class a region of
   // capacity = number of candidate quartets, for FP64 and (on demand) FP32
   std::vector<long long> q_off, q_cap;
@@ -269,8 +280,6 @@ struct mmdg_context {
   int total_keys = 0;
   DevBuf<long long> d_keyoff;
   DevBuf<int> d_keyw;  // primitive quartets of a quartet of the bucket
-  DevBuf<unsigned> d_qn;  // [2*total_keys]: FP64 and FP32 bucket lengths
-  DevBuf<unsigned long long> d_work;  // [2*MMDG_NCLASS]: work counters of the FP64 and FP32 class launches
   Geometry geom() const {
     Geometry g;
     g.pP = d_pP.p;
@@ -506,6 +515,21 @@ static int schwarz_lanes(int most) {
   return lg;
 }
 
+// largest Q of every tile of the class lists, from the current pair bounds
+static_assert(kPairClasses == (MMDG_LMAX + 1) * (MMDG_LMAX + 2) / 2, "pair classes");
+static cudaError_t tile_bounds(mmdg_context* h) {
+  TileArgs a;
+  int most = 0;
+  for (int c = 0; c < kNumPairClasses; ++c) {
+    a.list[c] = h->d_cls[c].p;
+    a.n[c] = h->cls_count[c];
+    a.qtile[c] = h->d_qtile[c].p;
+    most = std::max(most, a.n[c]);
+  }
+  k_tile_q<<<dim3((most + kThreads - 1) / kThreads, kNumPairClasses), kThreads>>>(a, h->d_Q.p);
+  return cudaGetLastError();
+}
+
 extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, int nshell, const int* shell_mol,
                               const int* shell_L, const int* shell_nprim, const double* shell_center,
                               const double* prim_exp, const double* prim_coef, const int* shell_func) {
@@ -615,8 +639,7 @@ extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, i
             h->d_pPf.alloc(2 * npp) == cudaSuccess && h->d_E64.alloc(ne) == cudaSuccess &&
             h->d_E32.alloc(ne) == cudaSuccess && h->d_Q.alloc(h->npair) == cudaSuccess &&
             h->d_screen.alloc(tt) == cudaSuccess && h->d_sq.alloc(tt) == cudaSuccess &&
-            h->d_sqf.alloc(tt) == cudaSuccess && h->d_dPf.alloc(nn) == cudaSuccess &&
-            h->d_Dsh.alloc(ss) == cudaSuccess && h->d_counters.alloc(kCounters * MMDG_NCLASS) == cudaSuccess;
+            h->d_sqf.alloc(tt) == cudaSuccess && h->d_Dsh.alloc(ss) == cudaSuccess;
   if (!ok) return fail(MMDG_E_NOMEM, "mmdg_set_basis: device allocation failed");
   // ---- primitive pairs
   {
@@ -829,7 +852,8 @@ extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, i
       h->group_start[c][gs[i]] = (int)i;
       h->group_prims[c][gs[i]] = std::max(h->group_prims[c][gs[i]], h->pr_count[v[i]]);
     }
-    if (h->d_gslot[c].upload(gs) != cudaSuccess) return fail(MMDG_E_NOMEM, "mmdg_set_basis: allocation");
+    if (h->d_gslot[c].upload(gs) != cudaSuccess ||
+        h->d_qtile[c].alloc((v.size() + kThreads - 1) / kThreads) != cudaSuccess) return fail(MMDG_E_NOMEM, "mmdg_set_basis: allocation");
     slot_group[c] = gs;
     slot_mol[c] = ms;
   }
@@ -869,6 +893,7 @@ extern "C" int mmdg_set_basis(mmdg_context* h, int nmol, const int* mol_nfunc, i
   h->q_off.clear();
   h->d_q64.release();
   h->d_q32.release();
+  CUDA_TRY(tile_bounds(h));
   CUDA_TRY(cudaDeviceSynchronize());
   h->have_basis = true;
   return MMDG_OK;
@@ -886,11 +911,11 @@ extern "C" int mmdg_device_bytes(mmdg_context* h, long long* bytes) {
   MMDG_ADD(d_mol_base); MMDG_ADD(d_mol_sbase); MMDG_ADD(d_mol_tbase); MMDG_ADD(d_mol_n); MMDG_ADD(d_mol_ns);
   MMDG_ADD(d_pa); MMDG_ADD(d_pb); MMDG_ADD(d_prb); MMDG_ADD(d_prc); MMDG_ADD(d_eoff);
   MMDG_ADD(d_pP); MMDG_ADD(d_pPf); MMDG_ADD(d_E64); MMDG_ADD(d_E32); MMDG_ADD(d_Q);
-  MMDG_ADD(d_mol_shell0); MMDG_ADD(d_screen); MMDG_ADD(d_sq); MMDG_ADD(d_sqf); MMDG_ADD(d_dPf); MMDG_ADD(d_Dsh);
-  MMDG_ADD(d_counters); MMDG_ADD(d_q64); MMDG_ADD(d_q32); MMDG_ADD(d_keyoff); MMDG_ADD(d_keyw); MMDG_ADD(d_qn); MMDG_ADD(d_work);
+  MMDG_ADD(d_mol_shell0); MMDG_ADD(d_screen); MMDG_ADD(d_sq); MMDG_ADD(d_sqf); MMDG_ADD(d_Dsh);
+  MMDG_ADD(d_zero); MMDG_ADD(d_screens); MMDG_ADD(d_q64); MMDG_ADD(d_q32); MMDG_ADD(d_keyoff); MMDG_ADD(d_keyw);
   MMDG_ADD(d_pair_owner); MMDG_ADD(d_pair_canon); MMDG_ADD(d_grad);
   for (int c = 0; c < kNumPairClasses; ++c) {
-    MMDG_ADD(d_cls[c]); MMDG_ADD(d_cls_moff[c]); MMDG_ADD(d_gslot[c]);
+    MMDG_ADD(d_cls[c]); MMDG_ADD(d_cls_moff[c]); MMDG_ADD(d_gslot[c]); MMDG_ADD(d_qtile[c]);
   }
 #undef MMDG_ADD
   *bytes = b;
@@ -936,7 +961,7 @@ extern "C" int mmdg_eri_tensor(mmdg_context* h, double* out, void* stream) {
     const ClassEntry& e = kClasses[ci];
     const int cb = pair_class(e.la, e.lb), ck = pair_class(e.lc, e.ld);
     if (!h->cls_count[cb] || !h->cls_count[ck]) continue;
-    ClassLaunch cl{h->d_cls[cb].p, h->d_cls[ck].p, h->cls_count[cb], h->cls_count[ck], cb == ck, 0.f, 0.f};
+    ClassLaunch cl{h->d_cls[cb].p, h->d_cls[ck].p, h->cls_count[cb], h->cls_count[ck], cb == ck};
     TensorBuckets tb;
     tb.nbg = h->ngroup[cb];
     tb.nkg = h->ngroup[ck];
@@ -1031,14 +1056,9 @@ extern "C" int mmdg_eri_quartets(mmdg_context* h, long long n, const int* shells
 }
 
 // ------------------------------------------------------------------ Fock build
-__global__ void k_prep_density(const double* dP, float* dPf, long long n) {
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  dPf[i] = float(fabs(dP[i]));
-}
-
-// per-molecule S x S block maxima of |dP|: one thread per (molecule, shell, shell)
-__global__ void k_shell_dmax(const float* dPf, float* Dsh, const int* func, const int* L,
+// per-molecule S x S block maxima of |dP|, rounded to FP32, and the molecule's largest (zeroed
+// before): one thread per (molecule, shell, shell)
+__global__ void k_shell_dmax(const double* dP, float* Dsh, float* dmax, const int* func, const int* L,
                              const long long* mol_base, const int* mol_n, const long long* mol_sbase,
                              const int* mol_ns, const long long* mol_shell0, int nmol, long long total) {
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -1054,7 +1074,7 @@ __global__ void k_shell_dmax(const float* dPf, float* Dsh, const int* func, cons
   const long long loc = idx - mol_sbase[m];
   const int a = (int)(loc / S), b = (int)(loc % S);
   const int s1 = (int)(mol_shell0[m] + a), s2 = (int)(mol_shell0[m] + b);
-  const float* D = dPf + mol_base[m];
+  const double* D = dP + mol_base[m];
   const int n1 = (L[s1] + 1) * (L[s1] + 2) / 2, n2 = (L[s2] + 1) * (L[s2] + 2) / 2;
   float mx = 0.f;
   for (int x = 0; x < n1; ++x) {
@@ -1063,10 +1083,11 @@ __global__ void k_shell_dmax(const float* dPf, float* Dsh, const int* func, cons
     for (int y = 0; y < n2; ++y) {
       const int j = func[s2 * kMaxComp + y];
       if (j < 0) continue;
-      mx = fmaxf(mx, D[(long long)i * N + j]);
+      mx = fmaxf(mx, float(fabs(D[(long long)i * N + j])));
     }
   }
   Dsh[idx] = mx;
+  atomicMax(reinterpret_cast<int*>(dmax + m), __float_as_int(mx));  // non-negative: ordered as integers
 }
 
 static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, double fp32_below,
@@ -1092,20 +1113,9 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
   cudaStream_t st = (cudaStream_t)stream;
   const long long nn = h->ntot_nn;
   CUDA_TRY(cudaMemsetAsync(G, 0, sizeof(double) * nn, st));
-  CUDA_TRY(cudaMemsetAsync(h->d_counters.p, 0, sizeof(unsigned long long) * kCounters * MMDG_NCLASS, st));
-  k_prep_density<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(dP, h->d_dPf.p, nn);
-  CUDA_TRY(cudaGetLastError());
-  {
-    const long long n = h->ntot_ss;
-    k_shell_dmax<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(h->d_dPf.p, h->d_Dsh.p, h->d_func.p, h->d_L.p,
-                                                              h->d_mol_base.p, h->d_mol_n.p, h->d_mol_sbase.p,
-                                                              h->d_mol_ns.p, h->d_mol_shell0.p, h->nmol, n);
-    CUDA_TRY(cudaGetLastError());
-  }
   Geometry g = h->geom();
   FockArgs f;
   f.dP = dP;
-  f.dPf = h->d_dPf.p;
   f.G = G;
   f.sq = h->d_sq.p;
   f.sqf = h->d_sqf.p;
@@ -1149,10 +1159,28 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
     }
     h->q_total = tot;
     h->total_keys = nk;
-    if (h->d_q64.alloc(tot > 0 ? tot : 1) != cudaSuccess || h->d_qn.alloc(2 * (nk > 0 ? nk : 1)) != cudaSuccess ||
-        h->d_work.alloc(2 * MMDG_NCLASS) != cudaSuccess ||
+    h->dmax_words = ((size_t)h->nmol + 1) / 2;
+    if (h->d_q64.alloc(tot > 0 ? tot : 1) != cudaSuccess ||
+        h->d_zero.alloc((kCounters + 2) * MMDG_NCLASS + h->dmax_words + nk) != cudaSuccess ||
         h->d_keyoff.upload(koff.empty() ? std::vector<long long>{0} : koff) != cudaSuccess ||
         h->d_keyw.upload(kw.empty() ? std::vector<int>{1} : kw) != cudaSuccess) {
+      h->q_off.clear();
+      return fail(MMDG_E_NOMEM, "mmdg_fock: cannot allocate the quartet lists");
+    }
+    std::vector<ScreenClass> sc;
+    int blocks = 0;
+    for (int ci = 0; ci < MMDG_NCLASS; ++ci) {
+      const ClassEntry& e = kClasses[ci];
+      const int cb = pair_class(e.la, e.lb), ck = pair_class(e.lc, e.ld);
+      if (!h->cls_count[cb] || !h->cls_count[ck]) continue;
+      sc.push_back({h->d_cls[cb].p, h->d_cls[ck].p, h->d_cls_moff[ck].p, h->d_gslot[cb].p, h->d_gslot[ck].p,
+                    h->d_qtile[ck].p, h->d_keyoff.p + h->kbase[ci], h->q_off[ci], h->kbase[ci], h->ngroup[ck], cb == ck,
+                    blocks});
+      blocks += h->cls_count[cb];
+    }
+    h->nscreen = (int)sc.size();
+    h->screen_blocks = blocks;
+    if (h->d_screens.upload(sc) != cudaSuccess) {
       h->q_off.clear();
       return fail(MMDG_E_NOMEM, "mmdg_fock: cannot allocate the quartet lists");
     }
@@ -1161,13 +1189,26 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
     if (h->d_q32.alloc(h->q_total > 0 ? h->q_total : 1) != cudaSuccess)
       return fail(MMDG_E_NOMEM, "mmdg_fock: cannot allocate the FP32 quartet lists");
   }
-  CUDA_TRY(cudaMemsetAsync(h->d_qn.p, 0, sizeof(unsigned) * 2 * (h->total_keys > 0 ? h->total_keys : 1), st));
-  CUDA_TRY(cudaMemsetAsync(h->d_work.p, 0, sizeof(unsigned long long) * 2 * MMDG_NCLASS, st));
+  CUDA_TRY(cudaMemsetAsync(h->d_zero.p, 0, sizeof(unsigned long long) * h->d_zero.n, st));
+  {
+    const long long n = h->ntot_ss;
+    k_shell_dmax<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dP, h->d_Dsh.p, h->dmax(), h->d_func.p, h->d_L.p,
+                                                              h->d_mol_base.p, h->d_mol_n.p, h->d_mol_sbase.p,
+                                                              h->d_mol_ns.p, h->d_mol_shell0.p, h->nmol, n);
+    CUDA_TRY(cudaGetLastError());
+  }
+  unsigned* const n64 = h->lengths();
+  unsigned* const n32 = n64 + h->total_keys;
+  if (h->screen_blocks) {
+    k_screen<<<h->screen_blocks, kThreads, 0, st>>>(g, f, h->d_screens.p, h->nscreen, h->d_q64.p,
+                                                    split > 0.f ? h->d_q32.p : h->d_q64.p, n64, n32, split, h->dmax());
+    CUDA_TRY(cudaGetLastError());
+  }
   cudaEvent_t ev[2 * MMDG_NCLASS];
   if (class_ms)
     for (int k = 0; k < 2 * MMDG_NCLASS; ++k) CUDA_TRY(cudaEventCreate(&ev[k]));
-  // ---- screening and evaluation of every class; with several streams class c runs
-  // both on stream c mod n (fork / join on events), so classes overlap
+  // ---- evaluation of every class; with several streams class c runs on stream c mod n
+  // (fork / join on events), so classes overlap
   const int ns = class_ms ? 1 : h->nstreams;
   std::unique_lock<std::mutex> side(h->side_mu, std::defer_lock);
   if (ns > 1) {
@@ -1175,49 +1216,32 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
     CUDA_TRY(cudaEventRecord(h->fork_ev, st));
     for (int k = 0; k < ns; ++k) CUDA_TRY(cudaStreamWaitEvent(h->side[k], h->fork_ev, 0));
   }
-  int ci = 0;
-  for (const ClassEntry& e : kClasses) {
+  // small molecules: highest angular momentum first, whose few quartets are the longest chains
+  // ((H2O)4 6-31G** 1.21 -> 1.16 ms); large ones: the long lists first ((H2O)16 39.6, reversed
+  // 39.9; mixed 19.1, 19.4).  The line lies between 0.7 and 171 million candidates.
+  const bool chains_first = !class_ms && h->q_total < (4 << 20);
+  for (int k = 0; k < MMDG_NCLASS; ++k) {
+    const int ci = chains_first ? MMDG_NCLASS - 1 - k : k;
+    const ClassEntry& e = kClasses[ci];
     const int cb = pair_class(e.la, e.lb), ck = pair_class(e.lc, e.ld);
-    if (h->cls_count[cb] && h->cls_count[ck]) {
-      ClassLaunch cl{h->d_cls[cb].p, h->d_cls[ck].p, h->cls_count[cb], h->cls_count[ck], cb == ck, 0.f, split,
-                     h->d_cls_moff[ck].p};
-      QuartetLists ql{h->d_q64.p + h->q_off[ci],
-                      split > 0.f ? h->d_q32.p + h->q_off[ci] : nullptr,
-                      h->d_qn.p + h->kbase[ci],
-                      h->d_qn.p + h->total_keys + h->kbase[ci],
-                      h->d_keyoff.p + h->kbase[ci],
-                      h->d_gslot[cb].p,
-                      h->d_gslot[ck].p,
-                      h->ngroup[ck],
-                      h->nkeys[ci]};
-      k_screen<<<cl.nbra, kThreads, 0, ns > 1 ? h->side[ci % ns] : st>>>(g, f, cl, ql);
-      CUDA_TRY(cudaGetLastError());
-    }
-    ++ci;
-  }
-  ci = 0;
-  for (const ClassEntry& e : kClasses) {
-    const int cb = pair_class(e.la, e.lb), ck = pair_class(e.lc, e.ld);
-    f.counters = h->d_counters.p + kCounters * ci;
+    f.counters = h->counters() + kCounters * ci;
     cudaStream_t cs = ns > 1 ? h->side[ci % ns] : st;
     if (class_ms) CUDA_TRY(cudaEventRecord(ev[2 * ci], st));
     if (h->cls_count[cb] && h->cls_count[ck]) {
-      ClassLaunch cl{h->d_cls[cb].p, h->d_cls[ck].p, h->cls_count[cb], h->cls_count[ck], cb == ck, 0.f, split,
-                     h->d_cls_moff[ck].p};
+      ClassLaunch cl{h->d_cls[cb].p, h->d_cls[ck].p, h->cls_count[cb], h->cls_count[ck], cb == ck};
       const int kb = h->kbase[ci];
-      BucketList bl{h->d_q64.p + h->q_off[ci], h->d_qn.p + kb, h->d_keyoff.p + kb, h->d_keyw.p + kb, h->nkeys[ci]};
+      BucketList bl{h->d_q64.p + h->q_off[ci], n64 + kb, h->d_keyoff.p + kb, h->d_keyw.p + kb, h->nkeys[ci]};
       const int grid = h->class_grid[ci], blk = h->class_block[ci], item = h->class_item[ci];
-      f.work = h->d_work.p + 2 * ci;
+      f.work = h->work() + 2 * ci;
       CUDA_TRY(e.fock(0, g, f, cl, bl, grid, blk, item, cs));
       if (split > 0.f) {
-        f.work = h->d_work.p + 2 * ci + 1;
+        f.work = h->work() + 2 * ci + 1;
         bl.list = h->d_q32.p + h->q_off[ci];
-        bl.count = h->d_qn.p + h->total_keys + kb;
+        bl.count = n32 + kb;
         CUDA_TRY(e.fock(1, g, f, cl, bl, grid, blk, item, cs));
       }
     }
     if (class_ms) CUDA_TRY(cudaEventRecord(ev[2 * ci + 1], st));
-    ++ci;
   }
   if (ns > 1)
     for (int k = 0; k < ns; ++k) {
@@ -1231,7 +1255,7 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
     for (int k = 0; k < 2 * MMDG_NCLASS; ++k) cudaEventDestroy(ev[k]);
   }
   if (counts) {
-    CUDA_TRY(cudaMemcpyAsync(counts, h->d_counters.p, sizeof(unsigned long long) * kCounters * MMDG_NCLASS,
+    CUDA_TRY(cudaMemcpyAsync(counts, h->counters(), sizeof(unsigned long long) * kCounters * MMDG_NCLASS,
                              cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
   }
@@ -1351,6 +1375,7 @@ extern "C" int mmdg_set_screen(mmdg_context* h, const double* screen, long long 
   k_pair_q_from_screen<<<(h->npair + 127) / 128, 128>>>(h->d_screen.p, h->d_Q.p, h->d_pa.p, h->d_pb.p, h->d_L.p,
                                                         h->d_func.p, h->d_shmol.p, h->d_mol_tbase.p, h->npair);
   CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(tile_bounds(h));
   CUDA_TRY(cudaDeviceSynchronize());
   return MMDG_OK;
 }

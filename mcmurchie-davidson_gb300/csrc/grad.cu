@@ -776,7 +776,7 @@ cudaError_t mmdg_launch_rhf_gradient(const GradArgs& a, const Geometry& g, const
       for (int x = 0; x <= k.ngroup; ++x) tb.kstart[x] = k.start[x];                                            \
       for (int x = 0; x < b.ngroup; ++x) tb.bw[x] = b.prims[x];                                                 \
       for (int x = 0; x < k.ngroup; ++x) tb.kw[x] = k.prims[x];                                                 \
-      const ClassLaunch cl{b.list, k.list, b.n, k.n, LA == LC && LB == LD, 0.f, 0.f, nullptr};                  \
+      const ClassLaunch cl{b.list, k.list, b.n, k.n, LA == LC && LB == LD};                  \
       return launch_two<LA, LB, LC, LD>(a, g, cl, tb, a.work + ci, nstreams > 1 ? side[ci % nstreams] : st);    \
     }                                                                                                           \
     return cudaSuccess;                                                                                         \

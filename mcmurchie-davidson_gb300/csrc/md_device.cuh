@@ -555,7 +555,6 @@ constexpr int kCounters = 5;
 
 struct FockArgs {
   const double* dP;      // packed per-molecule N x N (density difference)
-  const float* dPf;      // FP32 copy of |dP| for screening
   double* G;             // packed per-molecule N x N, accumulated (unsymmetrised)
   const double* sq;      // sqrt(screen) per molecule-local function pair, packed N(N+1)/2
   const float* sqf;      // FP32 copy

@@ -1,10 +1,9 @@
 // md_kernels.cuh -- the shell-quartet kernels (one instantiation per angular class).
 //
-// Fock builds (formPT semantics) run in two launches per angular class: k_screen
-// walks every candidate (bra shell pair, ket shell pair) of the class and appends
-// the survivors of the Schwarz x density bound to bucketed quartet lists (buckets
-// keyed by the primitive-count groups of the two pairs, FP64 and FP32 lists); then
-// k_fock, a persistent kernel, evaluates the list, 1 to 32 lanes per (quartet, ket
+// Fock builds (formPT semantics): k_screen walks the candidates (bra shell pair, ket
+// shell pair) of all angular classes and appends the survivors of the Schwarz x density bound to bucketed quartet lists (buckets
+// keyed by the primitive-count groups of the two pairs, FP64 and FP32 lists); then per
+// class k_fock, a persistent kernel, evaluates the list, 1 to 32 lanes per (quartet, ket
 // chunk) (the lanes share the quartet's primitive pairs, see plan_buckets),
 // chunk-major, so a warp shares its code path and, inside a bucket, its primitive
 // trip counts.  FP32 lists are split by grid stride; FP64 lists are claimed 32 lanes per
@@ -26,8 +25,6 @@ struct ClassLaunch {
   const int* ket;   // shell-pair indices of the ket class list
   int nbra, nket;
   int same;         // bra class == ket class: only ket slot <= bra slot
-  float qmin, qmax; // screening pass: quartets with Q_bra*Q_ket < qmax go to the FP32 list
-  const int* kmoff; // ket list: slot offset of every molecule (lists are molecule-major)
 };
 
 __host__ __device__ constexpr int ncart(int l) { return (l + 1) * (l + 2) / 2; }
@@ -51,22 +48,22 @@ __device__ __forceinline__ Ctx<Real> make_ctx(const Geometry& g, int bp, int kp,
   return c;
 }
 
-// Screening pass of one class pair: every candidate (bra slot, ket slot) is tested
-// against the shell-level bound Q_ab Q_cd max(4D_ab, 4D_cd, D_ac, D_ad, D_bc, D_bd)
-// (an upper bound of formPT's function-level test, fock.pyx:46-57) and appended to
-// the FP64 or the FP32 list of the class.  Each list is split into buckets keyed by
-// (bra primitive-count group, ket primitive-count group), so that the 32 quartets a
-// warp evaluates together have the same primitive loop trip counts.
-struct QuartetLists {
-  int2* q64;                  // class region (FP64)
-  int2* q32;                  // class region (FP32) or null
-  unsigned* n64;              // bucket lengths [nkeys]
-  unsigned* n32;
-  const long long* key_off;   // bucket offsets within the class region [nkeys]
-  const int* gbra;            // slot -> primitive-count group, bra class list
-  const int* gket;            // same for the ket class list
-  int nkg;                    // groups of the ket class list
-  int nkeys;
+// Screening pass of all classes: every candidate (bra slot, ket slot) is tested against
+// the shell-level bound Q_ab Q_cd max(4D_ab, 4D_cd, D_ac, D_ad, D_bc, D_bd) (an upper
+// bound of the function-level test, fock.pyx:46-57) and appended to the FP64 or the FP32
+// list of its class.  Each list is split into buckets keyed by (bra primitive-count
+// group, ket primitive-count group), so that the 32 quartets a warp evaluates together
+// have the same primitive loop trip counts.
+struct ScreenClass {
+  const int *bra, *ket;       // class lists
+  const int* kmoff;           // ket list: slot offset of every molecule (lists are molecule-major)
+  const int *gbra, *gket;     // slot -> primitive-count group
+  const float* qtile;         // largest Q of every kThreads ket slots
+  const long long* key_off;   // bucket offsets within the class region
+  long long region;           // first entry of the class in the quartet lists
+  int key0, nkg;              // first bucket, groups of the ket list
+  int same;                   // bra class == ket class: only ket slot <= bra slot
+  int first;                  // its first block
 };
 
 __device__ __forceinline__ void bucket_append(bool keep, int key, int2 v, int2* out, unsigned* n,
@@ -82,49 +79,99 @@ __device__ __forceinline__ void bucket_append(bool keep, int key, int2 v, int2* 
   out[key_off[key] + base + __popc(peers & ((1u << lane) - 1u))] = v;
 }
 
-// One block per bra slot; its threads walk the ket slots of the same molecule (the
+// One block per (class, bra slot); its threads walk the ket slots of the same molecule (the
 // lists are molecule-major), so a batch of molecules never forms cross-molecule
-// candidates.
-static __global__ void __launch_bounds__(kThreads) k_screen(Geometry g, FockArgs f, ClassLaunch cl, QuartetLists ql) {
-  const int ib = blockIdx.x;
-  if (ib >= cl.nbra) return;
-  const int bp = __ldg(cl.bra + ib);
+// candidates.  Tiles of kThreads kets whose largest Q cannot reach the threshold even with
+// the molecule's largest density element are passed over unread (most of a big molecule's:
+// the lists are sorted by Q inside a primitive-count group).  (H2O)16 6-31G**, all 21
+// classes: 0.6 ms; one launch per class, every candidate read, took 1.7.
+static __global__ void __launch_bounds__(kThreads) k_screen(Geometry g, FockArgs f, const ScreenClass* classes, int nclass,
+                                                            int2* q64, int2* q32, unsigned* n64, unsigned* n32,
+                                                            float split, const float* dmax) {
+  __shared__ unsigned s_tiles[kThreads / 32];
+  int lo = 0, hi = nclass - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (classes[mid].first <= (int)blockIdx.x) lo = mid;
+    else hi = mid - 1;
+  }
+  const ScreenClass c = classes[lo];
+  const int ib = (int)blockIdx.x - c.first;
+  const int bp = __ldg(c.bra + ib);
   const int sa = __ldg(g.pa + bp), sb = __ldg(g.pb + bp);
   const int mol = __ldg(g.sh_mol + sa);
   const float qb = __ldg(g.Q + bp);
-  const int gb = __ldg(ql.gbra + ib);
+  const int gb = __ldg(c.gbra + ib);
   const float* D = f.Dsh + g.mol_sbase[mol];
   const int S = g.mol_ns[mol];
   const int a = __ldg(g.sh_local + sa), b = __ldg(g.sh_local + sb);
   const float dab = 4.0f * __ldg(D + a * S + b);
-  const int k0 = __ldg(cl.kmoff + mol);
-  int k1 = __ldg(cl.kmoff + mol + 1);
-  if (cl.same) k1 = min(k1, ib + 1);
-  for (int base = k0; base < k1; base += kThreads) {
-    const int jk = base + threadIdx.x;
-    bool keep = jk < k1;
-    float qq = 0.f;
-    int key = 0;
-    if (keep) {
-      const int kp = __ldg(cl.ket + jk);
-      const int sc = __ldg(g.pa + kp), sd = __ldg(g.pb + kp);
-      qq = qb * __ldg(g.Q + kp);
-      const int c = __ldg(g.sh_local + sc), d = __ldg(g.sh_local + sd);
-      const float dm = fmaxf(fmaxf(dab, 4.0f * __ldg(D + c * S + d)),
-                             fmaxf(fmaxf(__ldg(D + a * S + c), __ldg(D + a * S + d)),
-                                   fmaxf(__ldg(D + b * S + c), __ldg(D + b * S + d))));
-      keep = qq * dm >= f.tolf_lo;
-      if (f.pair_owner) {
-        const int own = __ldg(f.pair_canon + bp) >= __ldg(f.pair_canon + kp) ? __ldg(f.pair_owner + bp)
-                                                                              : __ldg(f.pair_owner + kp);
-        keep = keep && own == f.part;
+  const float most = 4.0f * dmax[mol];
+  const int k0 = __ldg(c.kmoff + mol);
+  int k1 = __ldg(c.kmoff + mol + 1);
+  if (c.same) k1 = min(k1, ib + 1);
+  n64 += c.key0;
+  n32 += c.key0;
+  q64 += c.region;
+  q32 += c.region;
+  const int t1 = (k1 + kThreads - 1) / kThreads;
+  for (int t0 = k0 / kThreads; t0 < t1; t0 += kThreads) {
+    const int mine = t0 + threadIdx.x;
+    const bool open = mine < t1 && !((qb * __ldg(c.qtile + mine)) * most < f.tolf_lo);
+    const unsigned bits = __ballot_sync(0xffffffffu, open);
+    if ((threadIdx.x & 31) == 0) s_tiles[threadIdx.x >> 5] = bits;
+    __syncthreads();
+    for (int w = 0; w < kThreads / 32; ++w) {
+      for (unsigned left = s_tiles[w]; left; left &= left - 1) {
+        const int jk = (t0 + 32 * w + __ffs(left) - 1) * kThreads + threadIdx.x;
+        bool keep = jk >= k0 && jk < k1;
+        float qq = 0.f;
+        int key = 0;
+        if (keep) {
+          const int kp = __ldg(c.ket + jk);
+          const int sc = __ldg(g.pa + kp), sd = __ldg(g.pb + kp);
+          qq = qb * __ldg(g.Q + kp);
+          const int cc = __ldg(g.sh_local + sc), d = __ldg(g.sh_local + sd);
+          const float dm = fmaxf(fmaxf(dab, 4.0f * __ldg(D + cc * S + d)),
+                                 fmaxf(fmaxf(__ldg(D + a * S + cc), __ldg(D + a * S + d)),
+                                       fmaxf(__ldg(D + b * S + cc), __ldg(D + b * S + d))));
+          keep = qq * dm >= f.tolf_lo;
+          if (f.pair_owner) {
+            const int own = __ldg(f.pair_canon + bp) >= __ldg(f.pair_canon + kp) ? __ldg(f.pair_owner + bp)
+                                                                                  : __ldg(f.pair_owner + kp);
+            keep = keep && own == f.part;
+          }
+          key = gb * c.nkg + __ldg(c.gket + jk);
+        }
+        const bool low = qq < split;  // 0: no FP32 list
+        const int2 v = make_int2(ib, jk);
+        bucket_append(keep && !low, key, v, q64, n64, c.key_off);
+        if (split > 0.f) bucket_append(keep && low, key, v, q32, n32, c.key_off);
       }
-      key = gb * ql.nkg + __ldg(ql.gket + jk);
     }
-    const bool lo = qq < cl.qmax;  // qmax carries the FP32 split (0: none)
-    const int2 v = make_int2(ib, jk);
-    bucket_append(keep && !lo, key, v, ql.q64, ql.n64, ql.key_off);
-    if (ql.q32) bucket_append(keep && lo, key, v, ql.q32, ql.n32, ql.key_off);
+    __syncthreads();
+  }
+}
+
+// largest Q of every kThreads slots of the pair-class lists (blockIdx.y)
+constexpr int kPairClasses = 6;
+struct TileArgs {
+  const int* list[kPairClasses];
+  int n[kPairClasses];
+  float* qtile[kPairClasses];
+};
+static __global__ void __launch_bounds__(kThreads) k_tile_q(TileArgs a, const float* Q) {
+  __shared__ int s_q[kThreads / 32];
+  const int c = blockIdx.y, x = blockIdx.x * kThreads + threadIdx.x;
+  if ((int)blockIdx.x * kThreads >= a.n[c]) return;
+  const int q = x < a.n[c] ? __float_as_int(Q[a.list[c][x]]) : 0;  // Q >= 0: ordered as integers
+  const int m = __reduce_max_sync(0xffffffffu, q);
+  if ((threadIdx.x & 31) == 0) s_q[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int v = s_q[0];
+    for (int w = 1; w < kThreads / 32; ++w) v = max(v, s_q[w]);
+    a.qtile[c][blockIdx.x] = __int_as_float(v);
   }
 }
 

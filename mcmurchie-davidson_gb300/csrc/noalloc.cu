@@ -352,7 +352,7 @@ extern "C" int mmdg_eri_tensor_noalloc(int nshell, const int* shell_L, const int
     const int cb = ce.la * (ce.la + 1) / 2 + ce.lb, ck = ce.lc * (ce.lc + 1) / 2 + ce.ld;
     const int nb = lbeg[cb + 1] - lbeg[cb], nk = lbeg[ck + 1] - lbeg[ck];
     if (!nb || !nk) continue;
-    ClassLaunch cl{dlist + lbeg[cb], dlist + lbeg[ck], nb, nk, cb == ck, 0.f, 0.f};
+    ClassLaunch cl{dlist + lbeg[cb], dlist + lbeg[ck], nb, nk, cb == ck};
     TensorBuckets tb;
     tb.nbg = na_groups(prc, lists + lbeg[cb], nb, tb.bstart, tb.bw);
     tb.nkg = na_groups(prc, lists + lbeg[ck], nk, tb.kstart, tb.kw);
