@@ -71,24 +71,35 @@ def shells_from_bfs(bfs) -> ShellSet:
     angular momentum, exponents and component-free weights form one shell; any
     function that does not fit starts a new shell (its other components absent)."""
     L_, K_, cen_, ex_, co_, fn_ = [], [], [], [], [], []
-    cur = None  # (origin, L, exps, weights, last component index)
+    kinds: dict = {}   # function kind (component, exponents, weights) -> its number and data
+    joins: dict = {}   # (shell's first kind, its last component, kind) -> whether the function joins
+    origin0 = first = last = None  # the current shell: origin, kind of its first function, last component
     for f, b in enumerate(bfs):
-        lmn = tuple(int(x) for x in np.asarray(b.shell))
-        L = sum(lmn)
-        if L > LMAX:
-            raise ValueError(f"basis function {f} has angular momentum {L}; the GPU path supports up to {LMAX} (d)")
-        c = _COMP_INDEX[L][lmn]
         k = int(b.num_exps)
+        shell, exps = np.asarray(b.shell), np.asarray(b.exps, dtype=np.float64)[:k]
+        norm = np.asarray(b.norm, dtype=np.float64)[:k]
+        coefs = np.asarray(b.coefs, dtype=np.float64)[:k]
+        key = (shell.tobytes(), shell.dtype.char, exps.tobytes(), norm.tobytes(), coefs.tobytes())
+        kind = kinds.get(key)
+        if kind is None:  # a molecule has a few dozen kinds, each shared by many functions
+            lmn = tuple(int(x) for x in shell)
+            L = sum(lmn)
+            if L > LMAX:
+                raise ValueError(f"basis function {f} has angular momentum {L}; the GPU path supports up to {LMAX} (d)")
+            kind = kinds[key] = (len(kinds), L, _COMP_INDEX[L][lmn], exps, norm * coefs / comp_norm(lmn))
+        number, L, c, exps, w = kind
         origin = np.asarray(b.origin, dtype=np.float64).reshape(3)
-        exps = np.asarray(b.exps, dtype=np.float64)[:k]
-        w = np.asarray(b.norm, dtype=np.float64)[:k] * np.asarray(b.coefs, dtype=np.float64)[:k] / comp_norm(lmn)
-        # (the weights test is np.allclose(cur_w, w, rtol=1e-12, atol=0) written out)
-        join = (cur is not None and cur[1] == L and c > cur[4] and cur[2].shape == exps.shape
-                and bool((cur[0] == origin).all()) and bool((cur[2] == exps).all())
-                and bool((np.abs(cur[3] - w) <= 1e-12 * np.abs(w)).all()))
+        join = first is not None and bool((origin0 == origin).all())
+        if join:
+            pair = (first[0], last, number)
+            join = joins.get(pair)
+            if join is None:
+                _, L0, _, e0, w0 = first
+                # (the weights test is np.allclose(w0, w, rtol=1e-12, atol=0) written out)
+                join = joins[pair] = (L0 == L and c > last and e0.shape == exps.shape and bool((e0 == exps).all())
+                                      and bool((np.abs(w0 - w) <= 1e-12 * np.abs(w)).all()))
         if join:
             fn_[-1][c] = f
-            cur = (cur[0], cur[1], cur[2], cur[3], c)
         else:
             L_.append(L)
             K_.append(k)
@@ -98,7 +109,8 @@ def shells_from_bfs(bfs) -> ShellSet:
             row = np.full(MAX_COMP, -1, dtype=np.int32)
             row[c] = f
             fn_.append(row)
-            cur = (origin, L, exps, w, c)
+            origin0, first = origin, kind
+        last = c
     return ShellSet(nfunc=len(bfs), L=np.array(L_, dtype=np.int32), nprim=np.array(K_, dtype=np.int32),
                     center=np.array(cen_, dtype=np.float64).reshape(-1, 3),
                     exps=np.concatenate(ex_) if ex_ else np.zeros(0),
@@ -108,6 +120,6 @@ def shells_from_bfs(bfs) -> ShellSet:
 
 def fingerprint(bfs) -> tuple:
     """Cheap identity of a basis list (origins, shells, exponents, weights)."""
-    return tuple((tuple(np.asarray(b.origin, dtype=np.float64).tolist()), tuple(int(x) for x in b.shell),
-                  tuple(np.asarray(b.exps, dtype=np.float64).tolist()),
-                  tuple(np.asarray(b.coefs, dtype=np.float64).tolist())) for b in bfs)
+    return tuple((np.asarray(b.origin, dtype=np.float64).tobytes(), np.asarray(b.shell, dtype=np.int64).tobytes(),
+                  np.asarray(b.exps, dtype=np.float64).tobytes(), np.asarray(b.coefs, dtype=np.float64).tobytes())
+                 for b in bfs)
