@@ -238,13 +238,20 @@ __global__ void __launch_bounds__(256) k_mse(const float* __restrict__ Y, const 
                                              const double* __restrict__ count) {
   __shared__ double part[8];
   if (count) inv_count = (float)(1.0 / fmax((double)(float)*count, 1.0));
+  // 32 neighbours are summed in FP32, the rest in FP64: the loss's rounding does not depend on
+  // the grid
   double l = 0.0;
-  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
-    const float d = (Y[i] - T[i]) * mask[i];
-    dY[i] = 2.f * d * inv_count;
-    l += (double)(d * d * inv_count);
+  for (long long w = blockIdx.x * 256LL + (threadIdx.x & ~31); w < n; w += gridDim.x * 256LL) {
+    const long long i = w + (threadIdx.x & 31);
+    float q = 0.f;
+    if (i < n) {
+      const float d = (Y[i] - T[i]) * mask[i];
+      dY[i] = 2.f * d * inv_count;
+      q = d * d * inv_count;
+    }
+    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    l += (double)q;
   }
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = l;
   __syncthreads();
   if (threadIdx.x == 0) {

@@ -51,3 +51,25 @@ def test_linear_back_and_weight_gradient(rows, out, inp):
     e = (Y.double() - T.double()) * M.double()
     assert abs(float(loss) - float((e ** 2).sum()) / c) < 1e-6 * float((e ** 2).sum()) / c + 1e-12
     assert float(torch.linalg.norm(dY.double() - 2 * e / c)) < 1e-6 * float(torch.linalg.norm(2 * e / c)) + 1e-12
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 4097, 8192 * 81])
+def test_loss_sums_32_neighbours_in_fp32(n):
+    import torch
+    from mmd import _native
+    from mmd.guess import DensityMLP
+    L = _native.lib()
+    DensityMLP._sig(L)
+    rng = np.random.default_rng(n)
+    f = lambda: torch.as_tensor(rng.standard_normal(n).astype(np.float32), device="cuda")
+    Y, T, M = f(), f(), (f() > 0).float()
+    dY, loss = torch.empty_like(Y), torch.zeros(1, dtype=torch.float64, device="cuda")
+    inv = np.float32(1.0 / max(float(M.sum()), 1.0))
+    assert L.mmdg_mlp_mse(_p(Y), _p(T), _p(M), _p(dY), _p(loss), n, float(inv), _native.stream_ptr()) == 0
+    d = (Y - T) * M
+    q = torch.nn.functional.pad(d * d * float(inv), (0, -n % 32)).reshape(-1, 32)
+    while q.shape[1] > 1:
+        h = q.shape[1] // 2
+        q = q[:, :h] + q[:, h:]
+    # FP64 sums of positive terms in another order: 1e-16 a term, far inside 1e-12
+    assert abs(float(loss) - float(q.double().sum())) <= 1e-12 * float(loss) + 1e-300
