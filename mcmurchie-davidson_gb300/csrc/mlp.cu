@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdint>
 
 #include "../../include/mmdg.h"
 #include "pairs.cuh"
@@ -33,6 +34,13 @@ __device__ __forceinline__ float ld<__nv_bfloat16>(const __nv_bfloat16* p, long 
   return __bfloat162float(p[i]);
 }
 
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ld4(const __nv_bfloat16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);  // (a BF16 is the upper half of a float)
+  return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                     __uint_as_float(u.y & 0xffff0000u));
+}
+
 // What a GEMM does with its sums.
 enum Epilogue {
   kStore,   // C (+)= sums (atomics when K is split over blockIdx.z)
@@ -47,6 +55,23 @@ struct EpilogueArgs {
   int silu = 0;
 };
 
+// two FP32 FMAs in one instruction, each rounded as an FMA of its own
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long both(float x) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x));
+  return d;
+}
+__device__ __forceinline__ float2 halves(unsigned long long x) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(x));
+  return d;
+}
+
 __device__ __forceinline__ float silu_of(float z) { return z / (1.f + expf(-z)); }
 __device__ __forceinline__ float silu_grad(float z) {
   const float s = 1.f / (1.f + expf(-z));
@@ -54,13 +79,17 @@ __device__ __forceinline__ float silu_grad(float z) {
 }
 
 // op(A) op(B);  op(A): ta ? A^T (A stored K x M) : A (M x K), likewise B.  128 x 64 tiles, 8 x 4
-// outputs per thread read as float4 from shared memory (three 16-byte loads per 32 FMAs),
-// the next K stage in registers meanwhile.  Bound by FP32 issue (FMAs and the fetches'
-// index work) and, at the network's sizes, by the last wave: 256 tiles of an 8192 x 256
-// layer on 152 SMs.  With 64 x 64 tiles, 4 x 4 outputs and scalar shared loads the eight
-// GEMMs of a training step of 8192 rows took 840 us (7.7 TFLOP/s), now 300 (22).  Measured
-// per step: 128 x 64 tiles 363 us, 64 x 64 489, their K stage 8 or 32 deep 393 / 439.
-template <typename TA, typename TB, int EPI>
+// outputs per thread read as float4 from shared memory (three 16-byte loads per 32 FMAs, issued
+// as 16 packed pairs of rows), the next K stage in registers meanwhile.  VEC: rows of a
+// multiple of four elements at aligned addresses are fetched and written four at a time (78
+// registers against 128).  At the network's sizes it waits on latencies (ncu, 256 x 256 layer of
+// 8192 rows: FMA pipe 48 % busy, 3.3 warps per scheduler, stalls on the FMA chain, shared loads
+// and the fetch about equal) and on the last wave: 256 tiles on 152 SMs.  The eight GEMMs of a
+// training step of 8192 rows: 840 us with 64 x 64 tiles, 4 x 4 outputs and scalar shared loads,
+// 300 with these tiles, 290 with packed FMAs, 265 with fours (a 256 x 256 layer 45 -> 41 -> 37 us,
+// 29 TFLOP/s).  No better per step (320 us): 8 x 8 outputs per thread 332, two stages ahead in
+// registers 332, 64 x 64 tiles 334, both 429, K stages of 8 or 32 (before the fours) 393 / 439.
+template <typename TA, typename TB, int EPI, bool VEC>
 __global__ void __launch_bounds__(TT) k_gemm(int M, int N, int K, const TA* __restrict__ A, int lda, int ta,
                                               const TB* __restrict__ B, int ldb, int tb, float* __restrict__ C, int ldc,
                                               float beta, EpilogueArgs ep) {
@@ -84,6 +113,25 @@ __global__ void __launch_bounds__(TT) k_gemm(int M, int N, int K, const TA* __re
   };
   float ra[TK * TM / TT], rb[TK * TN / TT];
   auto fetch = [&](int k0) {
+    if (VEC) {  // four neighbours along the stored row at a time
+#pragma unroll
+      for (int x = 0; x < TK * TM / TT / 4; ++x) {
+        const int e = tid + x * TT;
+        const int m = m0 + (ta ? e % (TM / 4) * 4 : e / (TK / 4)), k = k0 + (ta ? e / (TM / 4) : e % (TK / 4) * 4);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (m < M && k < kend) v = ld4(ta ? A + (long long)k * lda + m : A + (long long)m * lda + k);
+        ra[4 * x] = v.x, ra[4 * x + 1] = v.y, ra[4 * x + 2] = v.z, ra[4 * x + 3] = v.w;
+      }
+#pragma unroll
+      for (int x = 0; x < TK * TN / TT / 4; ++x) {
+        const int e = tid + x * TT;
+        const int n = n0 + (tb ? e / (TK / 4) : e % (TN / 4) * 4), k = k0 + (tb ? e % (TK / 4) * 4 : e / (TN / 4));
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (n < N && k < kend) v = ld4(tb ? B + (long long)n * ldb + k : B + (long long)k * ldb + n);
+        rb[4 * x] = v.x, rb[4 * x + 1] = v.y, rb[4 * x + 2] = v.z, rb[4 * x + 3] = v.w;
+      }
+      return;
+    }
 #pragma unroll
     for (int x = 0; x < TK * TM / TT; ++x) {
       int kk, mm;
@@ -100,6 +148,31 @@ __global__ void __launch_bounds__(TT) k_gemm(int M, int N, int K, const TA* __re
     }
   };
   auto stage = [&](int s) {
+    if (VEC) {
+#pragma unroll
+      for (int x = 0; x < TK * TM / TT / 4; ++x) {
+        const int e = tid + x * TT;
+        if (ta) {
+          *reinterpret_cast<float4*>(&As[s][e / (TM / 4)][e % (TM / 4) * 4]) =
+              make_float4(ra[4 * x], ra[4 * x + 1], ra[4 * x + 2], ra[4 * x + 3]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) As[s][e % (TK / 4) * 4 + i][e / (TK / 4)] = ra[4 * x + i];
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < TK * TN / TT / 4; ++x) {
+        const int e = tid + x * TT;
+        if (!tb) {
+          *reinterpret_cast<float4*>(&Bs[s][e / (TN / 4)][e % (TN / 4) * 4]) =
+              make_float4(rb[4 * x], rb[4 * x + 1], rb[4 * x + 2], rb[4 * x + 3]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) Bs[s][e % (TK / 4) * 4 + i][e / (TK / 4)] = rb[4 * x + i];
+        }
+      }
+      return;
+    }
 #pragma unroll
     for (int x = 0; x < TK * TM / TT; ++x) {
       int kk, mm;
@@ -113,7 +186,7 @@ __global__ void __launch_bounds__(TT) k_gemm(int M, int N, int K, const TA* __re
       Bs[s][kk][nn] = rb[x];
     }
   };
-  float acc[8][4] = {};
+  unsigned long long acc2[4][4] = {};  // two rows each
   if (kbeg < kend) {
     fetch(kbeg);
     stage(0);
@@ -125,40 +198,69 @@ __global__ void __launch_bounds__(TT) k_gemm(int M, int N, int K, const TA* __re
     if (more) fetch(k0 + TK);
 #pragma unroll
     for (int kk = 0; kk < TK; ++kk) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[s][kk][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[s][kk][TM / 2 + ty * 4]);
+      const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(&As[s][kk][ty * 4]);
+      const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[s][kk][TM / 2 + ty * 4]);
       const float4 b0 = *reinterpret_cast<const float4*>(&Bs[s][kk][tx * 4]);
-      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, b[4] = {b0.x, b0.y, b0.z, b0.w};
+      const unsigned long long a[4] = {a0.x, a0.y, a1.x, a1.y}, b[4] = {both(b0.x), both(b0.y), both(b0.z), both(b0.w)};
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) acc2[i][j] = fma2(a[i], b[j], acc2[i][j]);
     }
     if (more) stage(s ^ 1);
     __syncthreads();
   }
-  float col[4] = {0.f, 0.f, 0.f, 0.f};
+  float acc[8][4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int m = m0 + (i < 4 ? 0 : TM / 2) + ty * 4 + (i & 3), n = n0 + tx * 4 + j;
-      if (m >= M || n >= N) continue;
-      const long long at = (long long)m * ldc + n;
+      const float2 v = halves(acc2[i][j]);
+      acc[2 * i][j] = v.x;
+      acc[2 * i + 1][j] = v.y;
+    }
+  float col[4] = {0.f, 0.f, 0.f, 0.f};
+  const int n = n0 + tx * 4;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int m = m0 + (i < 4 ? 0 : TM / 2) + ty * 4 + (i & 3);
+    if (m >= M || n >= N) continue;
+    const long long at = (long long)m * ldc + n;
+    if (VEC && (EPI != kStore || (gridDim.z == 1 && beta == 0.f))) {  // N a multiple of 4
+      float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
       if (EPI == kLinear) {
-        const float z = acc[i][j] + __ldg(ep.bias + n);
-        C[at] = z;
-        ep.Y[at] = ep.silu ? silu_of(z) : z;
+        const float4 q = ld4(ep.bias + n);
+        v = make_float4(v.x + q.x, v.y + q.y, v.z + q.z, v.w + q.w);
+        *reinterpret_cast<float4*>(ep.Y + at) =
+            ep.silu ? make_float4(silu_of(v.x), silu_of(v.y), silu_of(v.z), silu_of(v.w)) : v;
       } else if (EPI == kActGrad) {
-        const float d = ep.silu ? acc[i][j] * silu_grad(__ldg(ep.Zp + at)) : acc[i][j];
-        C[at] = d;
+        if (ep.silu) {
+          const float4 q = ld4(ep.Zp + at);
+          v = make_float4(v.x * silu_grad(q.x), v.y * silu_grad(q.y), v.z * silu_grad(q.z), v.w * silu_grad(q.w));
+        }
+        col[0] += v.x, col[1] += v.y, col[2] += v.z, col[3] += v.w;
+      }
+      *reinterpret_cast<float4*>(C + at) = v;
+      continue;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (n + j >= N) continue;
+      if (EPI == kLinear) {
+        const float z = acc[i][j] + __ldg(ep.bias + n + j);
+        C[at + j] = z;
+        ep.Y[at + j] = ep.silu ? silu_of(z) : z;
+      } else if (EPI == kActGrad) {
+        const float d = ep.silu ? acc[i][j] * silu_grad(__ldg(ep.Zp + at + j)) : acc[i][j];
+        C[at + j] = d;
         col[j] += d;
       } else if (gridDim.z > 1) {
-        atomicAdd(C + at, acc[i][j]);  // C zeroed by the launcher
+        atomicAdd(C + at + j, acc[i][j]);  // C zeroed by the launcher
       } else {
-        C[at] = beta != 0.f ? fmaf(beta, C[at], acc[i][j]) : acc[i][j];
+        C[at + j] = beta != 0.f ? fmaf(beta, C[at + j], acc[i][j]) : acc[i][j];
       }
     }
+  }
   if (EPI == kActGrad) {
     float* part = &As[0][0][0];  // [warp][column]: the K loop ended with a barrier
 #pragma unroll
@@ -299,6 +401,22 @@ int launch_fail(const char* what) {
 
 }  // namespace
 
+// whether every row of an operand can be read or written four elements at a time (else one by
+// one: 41 us against 37 for the layer above, whose sums are the same in the same order)
+template <typename T>
+static bool fours(const T* p, int ld, int inner) {
+  return p == nullptr || (ld % 4 == 0 && inner % 4 == 0 && reinterpret_cast<uintptr_t>(p) % (4 * sizeof(T)) == 0);
+}
+template <typename TA, typename TB, int EPI>
+static void gemm(dim3 grid, cudaStream_t st, int M, int N, int K, const TA* A, int lda, int ta, const TB* B, int ldb,
+                 int tb, float* C, int ldc, float beta, const EpilogueArgs& ep) {
+  if (fours(A, lda, ta ? M : K) && fours(B, ldb, tb ? K : N) && fours(C, ldc, N) && fours(ep.bias, 4, N) &&
+      fours(ep.Y, ldc, N) && fours(ep.Zp, ldc, N))
+    k_gemm<TA, TB, EPI, true><<<grid, TT, 0, st>>>(M, N, K, A, lda, ta, B, ldb, tb, C, ldc, beta, ep);
+  else
+    k_gemm<TA, TB, EPI, false><<<grid, TT, 0, st>>>(M, N, K, A, lda, ta, B, ldb, tb, C, ldc, beta, ep);
+}
+
 static const long long kFill = 304;  // blocks that fill the GPU: two per SM
 
 // C = op(A) op(B) (+ beta C): a_bf16 / b_bf16 select BF16 operands (weights)
@@ -321,14 +439,13 @@ extern "C" int mmdg_mlp_gemm(int M, int N, int K, const void* A, int lda, int ta
   }
   const EpilogueArgs ep;
   if (a_bf16 && !b_bf16)
-    k_gemm<__nv_bfloat16, float, kStore><<<grid, TT, 0, st>>>(M, N, K, (const __nv_bfloat16*)A, lda, ta,
-                                                               (const float*)B, ldb, tb, C, ldc, beta, ep);
+    gemm<__nv_bfloat16, float, kStore>(grid, st, M, N, K, (const __nv_bfloat16*)A, lda, ta, (const float*)B, ldb, tb, C,
+                                       ldc, beta, ep);
   else if (!a_bf16 && b_bf16)
-    k_gemm<float, __nv_bfloat16, kStore><<<grid, TT, 0, st>>>(M, N, K, (const float*)A, lda, ta,
-                                                               (const __nv_bfloat16*)B, ldb, tb, C, ldc, beta, ep);
+    gemm<float, __nv_bfloat16, kStore>(grid, st, M, N, K, (const float*)A, lda, ta, (const __nv_bfloat16*)B, ldb, tb, C,
+                                       ldc, beta, ep);
   else if (!a_bf16 && !b_bf16)
-    k_gemm<float, float, kStore><<<grid, TT, 0, st>>>(M, N, K, (const float*)A, lda, ta, (const float*)B, ldb, tb, C,
-                                                       ldc, beta, ep);
+    gemm<float, float, kStore>(grid, st, M, N, K, (const float*)A, lda, ta, (const float*)B, ldb, tb, C, ldc, beta, ep);
   else
     return mmdg_internal_fail(MMDG_E_ARG, "mmdg_mlp_gemm: at most one BF16 operand");
   return launch_fail("mmdg_mlp_gemm: launch");
@@ -345,8 +462,8 @@ extern "C" int mmdg_mlp_linear(long long rows, int out, int in, const float* X, 
   ep.Y = Y;
   ep.silu = silu;
   const dim3 grid((out + TN - 1) / TN, (unsigned)((rows + TM - 1) / TM));
-  k_gemm<float, __nv_bfloat16, kLinear><<<grid, TT, 0, (cudaStream_t)stream>>>(
-      (int)rows, out, in, X, in, 0, (const __nv_bfloat16*)W, in, 1, Z, out, 0.f, ep);
+  gemm<float, __nv_bfloat16, kLinear>(grid, (cudaStream_t)stream, (int)rows, out, in, X, in, 0, (const __nv_bfloat16*)W,
+                                      in, 1, Z, out, 0.f, ep);
   return launch_fail("mmdg_mlp_linear: launch");
 }
 
@@ -365,8 +482,8 @@ extern "C" int mmdg_mlp_back(long long rows, int out, int in, const float* dZ, c
   ep.db = db;
   ep.silu = silu;
   const dim3 grid((in + TN - 1) / TN, (unsigned)((rows + TM - 1) / TM));
-  k_gemm<float, __nv_bfloat16, kActGrad><<<grid, TT, 0, st>>>((int)rows, in, out, dZ, out, 0, (const __nv_bfloat16*)W,
-                                                               in, 0, dZp, in, 0.f, ep);
+  gemm<float, __nv_bfloat16, kActGrad>(grid, st, (int)rows, in, out, dZ, out, 0, (const __nv_bfloat16*)W, in, 0, dZp, in,
+                                       0.f, ep);
   return launch_fail("mmdg_mlp_back: launch");
 }
 

@@ -73,3 +73,33 @@ def test_loss_sums_32_neighbours_in_fp32(n):
         q = q[:, :h] + q[:, h:]
     # FP64 sums of positive terms in another order: 1e-16 a term, far inside 1e-12
     assert abs(float(loss) - float(q.double().sum())) <= 1e-12 * float(loss) + 1e-300
+
+
+@pytest.mark.parametrize("m,n,k", [(4, 4, 4), (128, 64, 16), (132, 68, 20), (260, 60, 100), (8, 256, 252)])
+def test_gemm_of_four_neighbours_equals_the_scalar_one(m, n, k):
+    """Packed rows of 4 elements take 16-byte loads; one element of padding or of offset does not."""
+    import torch
+    from mmd import _native
+    from mmd.guess import DensityMLP
+    L = _native.lib()
+    DensityMLP._sig(L)
+    st = _native.stream_ptr()
+    g = torch.Generator(device="cuda").manual_seed(m)
+    for a16, b16 in ((0, 0), (1, 0), (0, 1)):
+        for ta in (0, 1):
+            for tb in (0, 1):
+                A = torch.randn(*((k, m) if ta else (m, k)), generator=g, device="cuda")
+                B = torch.randn(*((n, k) if tb else (k, n)), generator=g, device="cuda")
+                A, B = A.bfloat16() if a16 else A, B.bfloat16() if b16 else B
+                out = []
+                for pad, off in ((0, 0), (1, 0), (0, 1)):
+                    args = []
+                    for x in (A, B):
+                        w = torch.zeros(x.shape[0] * (x.shape[1] + pad) + off, dtype=x.dtype, device="cuda")
+                        w[off:].view(x.shape[0], -1)[:, :x.shape[1]] = x
+                        args.append((w[off:], x.shape[1] + pad))
+                    C = torch.empty(m, n, device="cuda")
+                    assert L.mmdg_mlp_gemm(m, n, k, _p(args[0][0]), args[0][1], ta, a16, _p(args[1][0]), args[1][1], tb,
+                                           b16, _p(C), n, 0.0, st) == 0
+                    out.append(C)
+                assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])  # the same sums in the same order
