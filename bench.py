@@ -51,14 +51,14 @@ WORKLOAD = {"workload": "(H2O)16 6-31G** direct RHF", "n_water": 16, "lattice": 
 # the same rule and prints its own figure as config.fq_per_build).  Used by the
 # reference arm, which cannot run the 400-function SCF itself.
 FQ_PER_BUILD = 198282802.0
-# DRAM bytes (read + write) per launch of the dominant class kernel on this workload:
-# launch 5 of k_fock<MD_1000> (an early Fock build of the warm-up SCF) in one ncu capture
+# DRAM bytes (read + write) per launch of the two largest class kernels on this workload:
+# launch 5 of each (an early Fock build of the warm-up SCF) in one ncu capture
 # (dram__bytes_read.sum + dram__bytes_write.sum; summary and command in
 # profiles/k_fock_1000_full_h2o16.md).
-DRAM_BYTES_PER_LAUNCH = {"1000": 50.20e6}
+DRAM_BYTES_PER_LAUNCH = {"1000": 50.10e6, "1110": 16.26e6}
 # FP64-pipe busy fraction of the same launch over its elapsed cycles
 # (sm__pipe_fp64_cycles_active.avg.pct_of_peak_sustained_elapsed, same capture)
-FP64_PIPE_BUSY = {"1000": 0.846}
+FP64_PIPE_BUSY = {"1000": 0.819, "1110": 0.652}
 
 
 def _env():
