@@ -96,6 +96,7 @@ constexpr int kTcDigits = 8;
 constexpr int kTcStage = kTcRows * 16 * 2;          // bytes of one digit of a 16-wide k step
 constexpr int kTcTmem = kTcDigits * kTcCols;        // accumulator columns
 constexpr int kTcRawStride = 17;                    // doubles per row of the raw stage (16 + 1: no bank conflict)
+constexpr int kTcWide = 2 * kTcDigits - 1;          // digit slots of C per k octet: seven of zeros, then the digits
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -156,7 +157,7 @@ __device__ __forceinline__ uint32_t digit_pair(uint64_t u, uint64_t v, int i) {
   return __byte_perm(__float_as_uint(f), __float_as_uint(g), 0x7632u);
 }
 // eight consecutive k of one row: their digits as one 16-byte core-matrix row per digit
-__device__ __forceinline__ void store_digits(const double* x, int emax, unsigned char* at, int digit_bytes) {
+__device__ __forceinline__ void store_digits(const double* x, int emax, unsigned char* at) {
   uint32_t w[kTcDigits][4];
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
@@ -166,7 +167,7 @@ __device__ __forceinline__ void store_digits(const double* x, int emax, unsigned
   }
 #pragma unroll
   for (int i = 0; i < kTcDigits; ++i)
-    *reinterpret_cast<uint4*>(at + i * digit_bytes) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+    *reinterpret_cast<uint4*>(at + i * kTcStage) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
 }
 
 // the rare cases, kept out of line: a result outside the normal doubles, and a row or column
@@ -203,17 +204,18 @@ __device__ __forceinline__ double assemble(const uint32_t (*acc)[8], int col, in
   return __longlong_as_double((long long)(h == 0 ? 0ULL : (bits | (uint64_t)neg << 63)));
 }
 
-// One quarter transform.  Block (x, y): the S tile y (its digits of C stay in shared memory)
-// of the row tiles x, x + gridDim.x, ...  Per 16-wide k step the block stages the raw rows,
-// cuts them into digits and one thread issues the 36 digit products; two blocks per SM
+// One quarter transform.  Block (x, y): the S tile y (its part of C stays in shared memory as
+// 62-bit numbers: as digits it would take twice the room, one block per SM from N = 97 on) of
+// the row tiles x, x + gridDim.x, ...  Per 16-wide k step the block stages the raw rows, cuts
+// them and C's share into digits and one thread issues the digit products; two blocks per SM
 // (256 of the 512 TMEM columns each) overlap one's products with the other's digits.
-// Bound by the integer work around the products: of a tile's ~31,000 cycles at N = 76 (two
-// blocks per SM) about 6,600 cut digits, 7,400 put results together, 7,500 find the row
-// exponents and 6,000 stage rows; the tensor pipe is busy for 7 %.  One product of N =
-// (8 - i) NT columns per row digit i, instead of one per digit pair, took issuing them
-// from 2,400 to 150 cycles a step.  us per transform, k_quarter -> this: N = 7 86 -> 37,
-// 13 86 -> 43, 32 537 -> 77, 64 6,930 -> 926, 76 28,980 -> 2,720, 100 91,700 -> 10,400,
-// 128 219,500 -> 33,100 (FP64 arithmetic alone is 16,000 at N = 76, memory 320).
+// Bound by the integer work around the products: of a tile's ~34,000 cycles at N = 76 (two
+// blocks per SM) about 8,000 cut digits, 7,400 put results together, 7,500 find the row
+// exponents and 6,000 stage rows.  One product of N = 8 NT columns per row digit, instead of
+// one per digit pair, took issuing them from 2,400 to 150 cycles a step.  us per transform,
+// k_quarter -> this: N = 7 86 -> 34, 13 86 -> 41, 32 537 -> 81, 64 6,930 -> 1,020, 76
+// 28,980 -> 2,980, 100 91,700 -> 11,500, 128 219,500 -> 25,600 (FP64 arithmetic alone is
+// 16,000 at N = 76, memory 320).  C kept as digits: 76 2,915, 100 15,600, 128 38,000.
 // Prefetching the next tile into L2 was slower up to N = 76.
 __global__ void __launch_bounds__(kTcThreads, 2)
     k_quarter_tc(const double* __restrict__ in, const double* __restrict__ C, double* __restrict__ out, int N,
@@ -228,7 +230,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   const int S0 = blockIdx.y * kTcCols, cols = min(kTcCols, N - S0), NT = (cols + 15) & ~15;
   unsigned char* const As = sm;                                          // [digit][k octet][row][16 B]
   double* const raw = reinterpret_cast<double*>(sm + kTcDigits * kTcStage);
-  unsigned char* const Bs = sm + kTcDigits * kTcStage + sizeof(double) * kTcRawStride * kTcRows;  // [k octet][digit][S][16 B]
+  unsigned char* const Bs = sm + kTcDigits * kTcStage + sizeof(double) * kTcRawStride * kTcRows;  // [k octet][slot][S][16 B]
+  uint64_t* const Cf = reinterpret_cast<uint64_t*>(Bs + 2 * kTcWide * kTcCols * 16);              // [k octet][S][8]
   const uint32_t bar = smem_addr(&s_bar);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)),
@@ -240,7 +243,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  // ---- C's digits
+  // ---- C's fixed-point numbers, and the zeros before its digits
   for (int n = warp; n < kTcCols; n += kTcThreads / 32) {
     unsigned top = 0;
     if (n < cols)
@@ -253,16 +256,18 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   const uint32_t tmem = s_tmem;
   for (int u = tid; u < NT * (Kp / 8); u += kTcThreads) {
     const int n = u % NT, oct = u / NT;
-    double x[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int k = oct * 8 + j;
-      x[j] = n < cols && k < N ? __ldg(C + (long long)k * N + S0 + n) : 0.0;
+      Cf[u * 8 + j] = fixed_digits(n < cols && k < N ? __ldg(C + (long long)k * N + S0 + n) : 0.0, s_col[n]);
     }
-    store_digits(x, s_col[n], Bs + (oct * kTcDigits * NT + n) * 16, NT * 16);
   }
-  // instruction descriptor: D FP32, A and B BF16, both K-major, M (N is added per product)
-  const uint32_t idesc = 1u << 4 | 1u << 7 | 1u << 10 | (uint32_t)(kTcRows >> 4) << 24;
+  for (int u = tid; u < 2 * (kTcDigits - 1) * NT; u += kTcThreads) {
+    const int o = u / ((kTcDigits - 1) * NT);
+    *reinterpret_cast<uint4*>(Bs + (u + o * kTcDigits * NT) * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  // instruction descriptor: D FP32, A and B BF16, both K-major, N = 8 NT, M = 128
+  const uint32_t idesc = 1u << 4 | 1u << 7 | 1u << 10 | (uint32_t)(kTcDigits * NT >> 3) << 17 | (uint32_t)(kTcRows >> 4) << 24;
   uint32_t phase = 0;
   bool good = true;
   // largest exponent of every row of the tile at m: a warp per 16 rows, their loads in flight
@@ -320,21 +325,31 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         double x[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = raw[row * kTcRawStride + oct * 8 + j];
-        store_digits(x, s_row[row], As + (oct * kTcRows + row) * 16, kTcStage);
+        store_digits(x, s_row[row], As + (oct * kTcRows + row) * 16);
+        // C's digits of the step: a pair of k per thread
+        for (int u = tid; u < 8 * NT; u += kTcThreads) {
+          const ulonglong2 f = reinterpret_cast<const ulonglong2*>(Cf + (size_t)st * 16 * NT)[u];
+          const int o = u / (4 * NT);
+          unsigned char* const at = Bs + (o * kTcWide + kTcDigits - 1) * NT * 16 + (u - o * 4 * NT) * 4;
+#pragma unroll
+          for (int i = 0; i < kTcDigits; ++i) *reinterpret_cast<uint32_t*>(at + i * NT * 16) = digit_pair(f.x, f.y, i);
+        }
       }
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncthreads();
       if (tid == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         // the digits of C lie one after another along N, the accumulators one after another in
-        // TMEM: digit i of the rows meets digits 0 .. 7 - i of C in one product of N =
-        // (8 - i) NT columns, added into accumulators i .. 7
-        const uint32_t a0 = smem_addr(As);
-        const uint64_t b = operand(smem_addr(Bs) + (uint32_t)(st * 2 * kTcDigits * NT * 16), (uint32_t)(kTcDigits * NT * 16));
+        // TMEM: digit i of the rows meets digits 0 .. 7 - i of C, added into accumulators i .. 7.
+        // Every product spans all eight accumulators (its first i meet zeros): the ISA keeps
+        // tcgen05.mma of one thread in order for the same accumulator and shape only, and these
+        // all add into the same columns.
+        const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
 #pragma unroll
         for (int i = 0; i < kTcDigits; ++i)
-          mma_bf16(tmem + (uint32_t)(i * NT), operand(a0 + i * kTcStage, kTcRows * 16), b,
-                   idesc | (uint32_t)(((kTcDigits - i) * NT) >> 3) << 17, st > 0 || i > 0 ? 1u : 0u);
+          mma_bf16(tmem, operand(a0 + i * kTcStage, kTcRows * 16),
+                   operand(b0 + (uint32_t)((kTcDigits - 1 - i) * NT * 16), (uint32_t)(kTcWide * NT * 16)), idesc,
+                   st > 0 || i > 0 ? 1u : 0u);
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
                      : "memory");
       }
@@ -391,7 +406,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 // three, share an SM
 inline size_t tc_smem(int N) {
   const int Kp = (N + 15) / 16 * 16, NT = N < kTcCols ? (N + 15) / 16 * 16 : kTcCols;
-  const size_t need = (size_t)kTcDigits * kTcStage + sizeof(double) * kTcRawStride * kTcRows + (size_t)kTcDigits * Kp * NT * 2;
+  const size_t need = (size_t)kTcDigits * kTcStage + sizeof(double) * kTcRawStride * kTcRows + 2 * kTcWide * kTcCols * 16 +
+                      sizeof(uint64_t) * Kp * NT;
   return need < 80 * 1024 ? 80 * 1024 : need;
 }
 
@@ -421,9 +437,9 @@ extern "C" int mmdg_ao2mo(long long N, const double* C, const double* eri_in, do
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_quarter_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return mmdg_internal_fail(MMDG_E_CUDA, cudaGetErrorString(e));
-    const long long tiles = (M + kTcRows - 1) / kTcRows, per = smem <= 111 * 1024 ? 2 : 1;
+    const long long tiles = (M + kTcRows - 1) / kTcRows;
     tgrid.y = (unsigned)((N + kTcCols - 1) / kTcCols);
-    const long long want = per * sms / tgrid.y;
+    const long long want = 2LL * sms / tgrid.y;
     tgrid.x = (unsigned)(want < 1 ? 1 : (want < tiles ? want : tiles));
   }
   for (int q = 0; q < 4; ++q) {
