@@ -2125,7 +2125,6 @@ extern "C" int mmdg_rhf_gradient(mmdg_context* h, const double* P, const double*
       L.start[grp[x]] = (int)at;
       if (x + 1 == vals.size() || grp[x + 1] != grp[x]) L.prims[grp[x]] = vals[x];
     }
-    if ((long long)L.n * L.n > 0x7fffffffLL * 4) return fail(MMDG_E_ARG, "mmdg_rhf_gradient: too many shell pairs");
     // inside a group by Q: quartets below qtol end up together
     for (int x = 0; x < L.ngroup; ++x)
       std::stable_sort(v.begin() + L.start[x], v.begin() + L.start[x + 1], [&](int p, int q) { return Q[p] > Q[q]; });

@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kGradThreads) k_grad_two(GradArgs a, Geometry 
   constexpr bool DYN = B::L + K::L > 2;
   constexpr int U = DYN ? 1 : 256;
   constexpr bool STORE = NAB * 4 * HQ <= kGradStore;
-  __shared__ BucketPlan plan;
+  __shared__ BucketPlan<unsigned long long> plan;
   __shared__ typename GT::Data s_tab;
   static constexpr typename GT::Data ctab = GT::make();
   if constexpr (DYN)
@@ -342,7 +342,6 @@ __global__ void __launch_bounds__(kGradThreads) k_grad_two(GradArgs a, Geometry 
     if constexpr (DYN) return s_tab;
     else return ctab;
   }();
-  const unsigned n = plan.pre[nkeys];
   const int lane = threadIdx.x & 31;
   double* grad = a.grad + (long long)(blockIdx.x % kGradCopies) * 3 * a.natom;
   const int N = a.N;
@@ -351,11 +350,11 @@ __global__ void __launch_bounds__(kGradThreads) k_grad_two(GradArgs a, Geometry 
     unsigned long long base = 0;
     if (lane == 0) base = atomicAdd(work, 32ull);
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= n) break;
-    const unsigned r = (unsigned)base + lane;
+    if (base >= plan.pre[nkeys]) break;  // (kept in a register, it cost the d classes spills)
+    const unsigned long long r = base + lane;
     while (r >= plan.pre[x + 1]) ++x;
     const int lg = plan.lg[x], key = nkeys - 1 - x, wl = min(lg, 5);  // wl: the group's lanes in this warp
-    const unsigned slot = (r - plan.pre[x]) >> lg;
+    const unsigned long long slot = (r - plan.pre[x]) >> lg;
     if (slot >= bucket_quartets(tb, cl.same, key)) continue;
     int ib, jk;
     bucket_slot(tb, cl.same, key, slot, ib, jk);
@@ -365,7 +364,7 @@ __global__ void __launch_bounds__(kGradThreads) k_grad_two(GradArgs a, Geometry 
     // ---- this lane's share
     const int nb = __ldg(a.prc + bp), nk = __ldg(a.prc + kp);
     const int lgb = min(lg, 31 - __clz(nb)), lgk = min(lg - lgb, 31 - __clz(nk)), lga = lg - lgb - lgk;
-    const int sub = (int)((r - plan.pre[x]) & ((1u << lg) - 1u));
+    const int sub = (int)((unsigned)(r - plan.pre[x]) & ((1u << lg) - 1u));
     const int s0 = sub & ((1 << lgb) - 1), s1 = (sub >> lgb) & ((1 << lgk) - 1), s2 = sub >> (lgb + lgk);
     const int step = DYN ? 1 << lga : 1, ab0 = DYN ? s2 : 0;
     const int i0 = (s0 * nb) >> lgb, i1 = ((s0 + 1) * nb) >> lgb;

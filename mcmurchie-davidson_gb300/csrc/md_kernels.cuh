@@ -12,6 +12,7 @@
 // is screened), the Schwarz table runs a warp-wide group per heavy pair; listed
 // quartets use one thread per shell quartet.
 #pragma once
+#include "buckets.cuh"
 #include "md_device.cuh"
 #include "md_gen.cuh"
 
@@ -175,9 +176,6 @@ static __global__ void __launch_bounds__(kThreads) k_tile_q(TileArgs a, const fl
   }
 }
 
-constexpr int kMaxKeys = 256;
-constexpr int kMaxGroups = 16;  // primitive-count groups per pair-class list (kMaxGroups^2 <= kMaxKeys)
-
 // One bucketed list of a class: bucket k holds count[k] quartets from key_off[k] on, each
 // of about key_w[k] primitive quartets.
 struct BucketList {
@@ -190,9 +188,11 @@ struct BucketList {
 
 // How a launch walks its buckets: position x (heaviest bucket, stored last, first) covers
 // the work items pre[x] .. pre[x + 1), a multiple of 32, of bucket nkeys - 1 - x, with
-// 2^lg[x] lanes per quartet.
+// 2^lg[x] lanes per quartet.  Index: unsigned for the Fock lists, whose lengths are 32-bit
+// counters, 64 bits for the unscreened classes (buckets.cuh).
+template <typename Index>
 struct BucketPlan {
-  unsigned pre[kMaxKeys + 1];
+  Index pre[kMaxKeys + 1];
   unsigned char lg[kMaxKeys];
 };
 
@@ -209,8 +209,8 @@ struct BucketPlan {
 // 8 on (H2O)4: 2.45, 1.44, 1.33, 4 the better on one stream.  One thread per quartet: 2.74.
 constexpr float kLanePrims = 4.0f;
 
-template <class CountF, class WeightF>
-__device__ __forceinline__ void plan_buckets(BucketPlan& p, int nkeys, int nchunk, long long nthreads, CountF count,
+template <typename Index, class CountF, class WeightF>
+__device__ __forceinline__ void plan_buckets(BucketPlan<Index>& p, int nkeys, int nchunk, long long nthreads, CountF count,
                                              WeightF weight, int most = 5) {
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
@@ -218,20 +218,20 @@ __device__ __forceinline__ void plan_buckets(BucketPlan& p, int nkeys, int nchun
     for (int x = lane; x < nkeys; x += 32) W += float(count(nkeys - 1 - x)) * float(weight(nkeys - 1 - x));
     for (int o = 16; o > 0; o >>= 1) W += __shfl_xor_sync(0xffffffffu, W, o);
     const float share = fmaxf(kLanePrims, 2.0f * W * float(nchunk) / float(nthreads));
-    unsigned acc = 0;
+    Index acc = 0;
     for (int x0 = 0; x0 < nkeys; x0 += 32) {
       const int x = x0 + lane;
-      unsigned len = 0;
+      Index len = 0;
       int lg = 0;
       if (x < nkeys) {
-        const unsigned c = count(nkeys - 1 - x);
+        const Index c = count(nkeys - 1 - x);
         const float w = float(weight(nkeys - 1 - x));
         while (lg < most && w > share * float(1 << lg)) ++lg;
-        len = ((c << lg) + 31u) & ~31u;
+        len = bucket_items(c, lg);
       }
-      unsigned end = len;
+      Index end = len;
       for (int d = 1; d < 32; d <<= 1) {
-        const unsigned t = __shfl_up_sync(0xffffffffu, end, d);
+        const Index t = __shfl_up_sync(0xffffffffu, end, d);
         if (lane >= d) end += t;
       }
       if (x < nkeys) {
@@ -301,7 +301,7 @@ struct GroupDigest {
 // neighbouring quartets.
 template <class MD, typename Real>
 __global__ void __launch_bounds__(kMaxFockBlock) k_fock(Geometry g, FockArgs f, ClassLaunch cl, BucketList bl) {
-  __shared__ BucketPlan plan;
+  __shared__ BucketPlan<unsigned> plan;
   // block size: kThreads for classes with shared-memory R tables, else 64..256 (tile),
   // a multiple of 32 either way, so every warp is full
   const long long nthreads = (long long)gridDim.x * blockDim.x;
@@ -376,65 +376,31 @@ __global__ void __launch_bounds__(kMaxFockBlock) k_fock(Geometry g, FockArgs f, 
   }
 }
 
-// The buckets of an unscreened class of one molecule: its class lists are sorted by
-// primitive count, so group g of the bra list is the slots bstart[g] .. bstart[g + 1),
-// each of at most bw[g] primitive pairs; bucket k = gb * nkg + gk is the rectangle of two
-// groups (the triangle for a group with itself, nothing for gk > gb, when the lists are
-// the same).
-struct TensorBuckets {
-  int nbg, nkg;
-  int bstart[kMaxGroups + 1], kstart[kMaxGroups + 1];
-  int bw[kMaxGroups], kw[kMaxGroups];
-};
-
-// quartets of bucket k
-__device__ __forceinline__ unsigned bucket_quartets(const TensorBuckets& tb, int same, int k) {
-  const int gb = k / tb.nkg, gk = k - gb * tb.nkg;
-  const unsigned a = tb.bstart[gb + 1] - tb.bstart[gb], b = tb.kstart[gk + 1] - tb.kstart[gk];
-  return !same || gk < gb ? a * b : (gk == gb ? a * (a + 1) / 2 : 0u);
-}
-
-// bra and ket list slot of a bucket's quartet
-__device__ __forceinline__ void bucket_slot(const TensorBuckets& tb, int same, int key, unsigned slot, int& ib, int& jk) {
-  const int gb = key / tb.nkg, gk = key - gb * tb.nkg;
-  if (same && gb == gk) {  // slot = ib (ib + 1) / 2 + jk
-    ib = (int)((sqrtf(8.0f * float(slot) + 1.0f) - 1.0f) * 0.5f);
-    while ((long long)ib * (ib + 1) / 2 > (long long)slot) --ib;
-    while ((long long)(ib + 1) * (ib + 2) / 2 <= (long long)slot) ++ib;
-    jk = (int)((long long)slot - (long long)ib * (ib + 1) / 2);
-  } else {
-    const unsigned b = tb.kstart[gk + 1] - tb.kstart[gk];
-    ib = (int)(slot / b);
-    jk = (int)(slot - (unsigned)ib * b);
-  }
-  ib += tb.bstart[gb];
-  jk += tb.kstart[gk];
-}
-
 // Every ERI of the class into the tensor, 1 to 32 lanes per (quartet, ket chunk) as in
 // k_fock, persistent over the buckets.  (One thread per quartet: N = 75 10.6 ms, its 21
 // launches each as long as their heaviest quartet; with groups 2.2 ms one after another, the
 // classes on eight streams 1.15.)
 template <class MD>
 __global__ void __launch_bounds__(kThreads) k_tensor(Geometry g, TensorArgs t, ClassLaunch cl, TensorBuckets tb) {
-  __shared__ BucketPlan plan;
+  __shared__ BucketPlan<unsigned long long> plan;
   const int nkeys = tb.nbg * tb.nkg;
   plan_buckets(plan, nkeys, MD::NCHUNK, (long long)gridDim.x * kThreads,
                [&](int k) { return bucket_quartets(tb, cl.same, k); },
                [&](int k) { return tb.bw[k / tb.nkg] * tb.kw[k % tb.nkg]; });
-  const unsigned n = plan.pre[nkeys];
-  const long long total = (long long)n * MD::NCHUNK, stride = (long long)gridDim.x * kThreads;
+  // (64-bit totals kept in registers would cost the larger classes spills: read where needed)
+  const int stride = gridDim.x * kThreads;
   const unsigned lane = threadIdx.x & 31u;
   extern __shared__ double smem_d[];
   double* rs = smem_d + threadIdx.x;
   int x = 0;
-  for (long long idx = ((long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + lane; idx < total; idx += stride) {
-    const int chunk = (int)(idx / n);
-    const unsigned r = (unsigned)(idx - (long long)chunk * n);
+  for (long long idx = ((long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + lane;
+       idx < (long long)plan.pre[nkeys] * MD::NCHUNK; idx += stride) {
+    const int chunk = MD::NCHUNK > 1 ? (int)(idx / (long long)plan.pre[nkeys]) : 0;
+    const unsigned long long r = (unsigned long long)idx - chunk * plan.pre[nkeys];
     if (r < plan.pre[x]) x = 0;
     while (r >= plan.pre[x + 1]) ++x;
     const int lg = plan.lg[x], key = nkeys - 1 - x;
-    const unsigned slot = (r - plan.pre[x]) >> lg;
+    const unsigned long long slot = (r - plan.pre[x]) >> lg;
     if (slot >= bucket_quartets(tb, cl.same, key)) continue;
     int ib, jk;
     bucket_slot(tb, cl.same, key, slot, ib, jk);
