@@ -433,7 +433,8 @@ extern "C" int mmdg_mlp_gemm(int M, int N, int K, const void* A, int lda, int ta
     const int split = (int)std::min<long long>((K + 127) / 128, (kFill + tiles - 1) / tiles);
     if (split > 1) {
       grid.z = split;
-      if (cudaMemsetAsync(C, 0, sizeof(float) * (size_t)M * ldc, st) != cudaSuccess)
+      // the N columns alone: what lies between them and ldc is the caller's
+      if (cudaMemset2DAsync(C, sizeof(float) * std::max(ldc, N), 0, sizeof(float) * N, M, st) != cudaSuccess)
         return mmdg_internal_fail(MMDG_E_CUDA, "mmdg_mlp_gemm: memset");
     }
   }
