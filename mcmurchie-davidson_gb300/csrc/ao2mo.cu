@@ -435,7 +435,10 @@ extern "C" int mmdg_ao2mo(long long N, const double* C, const double* eri_in, do
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_quarter_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the kernel's limit belongs to the device, not to the call: always that of the largest N,
+    // so that no thread lowers it under another's launch)
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_quarter_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem((int)kTcMax));
     if (e != cudaSuccess) return mmdg_internal_fail(MMDG_E_CUDA, cudaGetErrorString(e));
     const long long tiles = (M + kTcRows - 1) / kTcRows;
     tgrid.y = (unsigned)((N + kTcCols - 1) / kTcCols);
