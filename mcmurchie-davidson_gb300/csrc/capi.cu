@@ -288,7 +288,9 @@ struct mmdg_context {
   int nstreams = 1;
   cudaStream_t side[kMaxStreams] = {};
   cudaEvent_t fork_ev = nullptr, join_ev[kMaxStreams] = {};
-  std::mutex side_mu;  // held while a call forks onto the side streams and joins them
+  // held while a call forks onto the side streams and joins them, and over a whole capture:
+  // the streams that a captured call forked onto stay in capture until it ends
+  std::recursive_mutex side_mu;
   // CUDA graph of one Fock build (mmdg_fock_graph)
   cudaGraphExec_t graph = nullptr;
   const double* g_dP = nullptr;
@@ -561,6 +563,21 @@ static int schwarz_lanes(int most) {
   int lg = 0;
   while (lg < 5 && (long long)most * most > (4LL << lg)) ++lg;
   return lg;
+}
+
+// How many side streams a call on st may fork onto (side_mu held): none while st is captured
+// or another thread's capture has the side streams, which every call shares.
+static int side_streams(mmdg_context* h, cudaStream_t st) {
+  if (h->nstreams < 2) return 1;
+  for (cudaStream_t x : {st, h->side[0]}) {  // (a fork takes all of them, the first included)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(x, &capture) != cudaSuccess) {
+      cudaGetLastError();
+      return 1;
+    }
+    if (capture != cudaStreamCaptureStatusNone) return 1;
+  }
+  return h->nstreams;
 }
 
 // largest Q of every tile of the class lists, from the current pair bounds
@@ -991,15 +1008,9 @@ extern "C" int mmdg_eri_tensor(mmdg_context* h, double* out, void* stream) {
   TensorArgs t{out};
   // the classes overlap on the context's streams (each launch ends in a tail of its heaviest
   // quartets: N = 25 on one stream 1.54 ms, on eight 0.30; N = 75 1.90, 1.13; N = 100 3.38,
-  // 2.62), highest angular momentum first.  A call that is being captured stays on its stream:
-  // the side streams are every caller's.
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
-    cudaGetLastError();
-    capture = cudaStreamCaptureStatusActive;
-  }
-  const int ns = capture == cudaStreamCaptureStatusNone ? h->nstreams : 1;
-  std::lock_guard<std::mutex> lock(h->side_mu);
+  // 2.62), highest angular momentum first.
+  std::lock_guard<std::recursive_mutex> lock(h->side_mu);
+  const int ns = side_streams(h, st);
   if (ns > 1) {
     CUDA_TRY(cudaEventRecord(h->fork_ev, st));
     for (int k = 0; k < ns; ++k) CUDA_TRY(cudaStreamWaitEvent(h->side[k], h->fork_ev, 0));
@@ -1257,7 +1268,7 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
   // ---- evaluation of every class; with several streams class c runs on stream c mod n
   // (fork / join on events), so classes overlap
   const int ns = class_ms ? 1 : h->nstreams;
-  std::unique_lock<std::mutex> side(h->side_mu, std::defer_lock);
+  std::unique_lock<std::recursive_mutex> side(h->side_mu, std::defer_lock);
   if (ns > 1) {
     side.lock();
     CUDA_TRY(cudaEventRecord(h->fork_ev, st));
@@ -2210,8 +2221,8 @@ extern "C" int mmdg_rhf_gradient(mmdg_context* h, const double* P, const double*
     first += gl[c].n;
   }
   {
-    std::lock_guard<std::mutex> side(h->side_mu);
-    CUDA_TRY(mmdg_launch_rhf_gradient(a, geo, gl, h->nstreams, h->side, h->fork_ev, h->join_ev, st));
+    std::lock_guard<std::recursive_mutex> side(h->side_mu);
+    CUDA_TRY(mmdg_launch_rhf_gradient(a, geo, gl, side_streams(h, st), h->side, h->fork_ev, h->join_ev, st));
   }
   std::vector<double> g(3 * (size_t)natom);
   CUDA_TRY(cudaMemcpyAsync(g.data(), a.grad, sizeof(double) * 3 * natom, cudaMemcpyDeviceToHost, st));
@@ -2318,9 +2329,13 @@ extern "C" int mmdg_fock_graph(mmdg_context* h, const double* dP, double* G, dou
     CUDA_TRY(cudaStreamSynchronize(st));
     if (!h->g_stream) CUDA_TRY(cudaStreamCreateWithFlags(&h->g_stream, cudaStreamNonBlocking));
     cudaGraph_t graph = nullptr;
-    CUDA_TRY(cudaStreamBeginCapture(h->g_stream, cudaStreamCaptureModeThreadLocal));
-    rc = fock_impl(h, dP, G, tol, fp32_below, nullptr, nullptr, h->g_stream);
-    cudaError_t e = cudaStreamEndCapture(h->g_stream, &graph);
+    cudaError_t e;
+    {
+      std::lock_guard<std::recursive_mutex> side(h->side_mu);
+      CUDA_TRY(cudaStreamBeginCapture(h->g_stream, cudaStreamCaptureModeThreadLocal));
+      rc = fock_impl(h, dP, G, tol, fp32_below, nullptr, nullptr, h->g_stream);
+      e = cudaStreamEndCapture(h->g_stream, &graph);
+    }
     if (rc) {
       if (graph) cudaGraphDestroy(graph);
       return rc;
