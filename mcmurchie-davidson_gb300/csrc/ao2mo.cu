@@ -13,15 +13,26 @@
 // a thread's 16 independent FMAs per k step cost nothing; the 16 accumulators keep
 // the pipe fed.
 //
-// Up to N = 128 the product runs on the tensor cores instead (k_quarter_tc), exactly
-// up to a rounding far below a double's: every row of the tensor and every column of C is
-// scaled by a power of two and cut into eight signed 8-bit digits (62 bits), digits are
-// exact BF16 numbers, and the digit products with i + j = d, d = 0..7 (36 of 64), are
-// summed by tcgen05.mma in one FP32 accumulator per d: at most 8 x 128 products of at
-// most 2^14, so every sum is an integer of at most 2^24 and exact.  The eight integers
-// are put together in fixed point and rounded once.  Left out are digit products below
-// 2^-62 of (row maximum) x (column maximum).  (Split-operand products after K. Ozaki,
-// T. Ogita, S. Oishi and S. M. Rump, Numer. Algorithms 59, 95-118, 2012.)
+// Up to N = 128 the product runs on the tensor cores instead (k_quarter_tc): every row of
+// the tensor and every column of C is scaled by a power of two and cut into eight signed
+// 8-bit digits (62 bits), digits are exact BF16 numbers, and the digit products with
+// i + j = d, d = 0..7 (36 of 64), are summed by tcgen05.mma in one FP32 accumulator per d:
+// at most 8 x 128 products of at most 2^14, so every sum is an integer of at most 2^24 and
+// exact.  The eight integers are put together in fixed point and rounded once.  (Split-
+// operand products after K. Ozaki, T. Ogita, S. Oishi and S. M. Rump, Numer. Algorithms 59,
+// 95-118, 2012.)
+//
+// Left out are the bits below a row's and a column's 62 and the digit products with i + j >
+// 7, together at most 9.03 units of 2^62 per k in the fixed-point product, whose unit is
+// 2^(er + ec - 2168) with er, ec the exponent fields of the row's and the column's largest
+// element: at most 9.03 N 2^(er + ec - 2106) (rms 2^-57 of their product at N = 76).  An FP64
+// sum may be off by N 2^-53 S, S = sum_k |a_k| |c_k|.  The first is the smaller bound where S
+// is at least 2^(er + ec - 2049), an eighth of the product of the two largest elements' powers
+// of two: 0.57 N 2^-53 S.  So an output is kept if it is that large itself, or if one of the
+// largest elements meets a partner that makes the product so; every other one (a weak one: the
+// largest elements meet small ones, as a localised or symmetry-adapted C over decaying rows) is
+// looked at along its row and column and, with no such product, summed in FP64.  No element is
+// less exact than an FP64 sum may be.
 #include <cuda_runtime.h>
 
 #include <stdint.h>
@@ -96,6 +107,8 @@ constexpr int kTcDigits = 8;
 constexpr int kTcStage = kTcRows * 16 * 2;          // bytes of one digit of a 16-wide k step
 constexpr int kTcTmem = kTcDigits * kTcCols;        // accumulator columns
 constexpr int kTcRawStride = 17;                    // doubles per row of the raw stage (16 + 1: no bank conflict)
+constexpr int kTcQueue = 256;                       // weak outputs looked at together
+constexpr int kTcMany = 512;                        // of a tile: from here on they are summed at once
 constexpr int kTcWide = 2 * kTcDigits - 1;          // digit slots of C per k octet: seven of zeros, then the digits
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -170,18 +183,19 @@ __device__ __forceinline__ void store_digits(const double* x, int emax, unsigned
     *reinterpret_cast<uint4*>(at + i * kTcStage) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
 }
 
-// the rare cases, kept out of line: a result outside the normal doubles, and a row or column
-// with an infinity or NaN (as plain arithmetic has it)
-__device__ __noinline__ double scaled(uint64_t mant, int e) { return ldexp((double)mant, e); }
-__device__ __noinline__ double plain_dot(const double* __restrict__ row, const double* __restrict__ C, int N) {
-  double v = 0.0;
-  for (int k = 0; k < N; ++k) v = fma(__ldg(row + k), __ldg(C + (long long)k * N), v);
-  return v;
-}
+// An element's size and place: the upper half of its magnitude with k (below 128) in the lowest
+// bits, so that a maximum over a row or column brings its exponent field and where it is
+__device__ __forceinline__ unsigned size_at(int hi, int k) { return ((unsigned)hi & 0x7fffff80u) | (unsigned)k; }
+__device__ __forceinline__ int field_of(unsigned size) { return (int)(size >> 20); }
+__device__ __forceinline__ unsigned at_least_one(unsigned size) { return field_of(size) ? size : size | 1u << 20; }
 
-// sum_d acc_d 256^(7-d) 2^scale as a double, rounded to nearest, without a branch (eight of
-// them interleave); outside the normal doubles `far` is set, and the value is (-1)^neg mant 2^e
-__device__ __forceinline__ double assemble(const uint32_t (*acc)[8], int col, int scale, bool& far, bool& neg,
+// the rare case, kept out of line: a result outside the normal doubles
+__device__ __noinline__ double scaled(uint64_t mant, int e) { return ldexp((double)mant, e); }
+
+// sum_d acc_d 256^(7-d) 2^(top - 2112) as a double, rounded to nearest, without a branch (eight
+// of them interleave); outside the normal doubles `far` is set, and the value is (-1)^neg mant
+// 2^e.  `low`: below 2^63 units, 2^(top - 2049).
+__device__ __forceinline__ double assemble(const uint32_t (*acc)[8], int col, int top_field, bool& far, bool& low, bool& neg,
                                            uint64_t& mant, int& e) {
   int a[kTcDigits];
 #pragma unroll
@@ -190,18 +204,106 @@ __device__ __forceinline__ double assemble(const uint32_t (*acc)[8], int col, in
   const long long lo = (long long)a[4] * (1 << 24) + ((long long)a[5] * (1 << 16) + ((long long)a[6] * (1 << 8) + a[7]));
   hi += lo >> 32;  // value = hi 2^32 + (low 32 bits of lo)
   neg = hi < 0;  // magnitude of the 96-bit two's complement number
-  const uint32_t low = neg ? 0u - (uint32_t)lo : (uint32_t)lo;
-  hi = neg ? ~hi + (low == 0u) : hi;
+  const uint32_t tail = neg ? 0u - (uint32_t)lo : (uint32_t)lo;
+  hi = neg ? ~hi + (tail == 0u) : hi;
+  low = (hi >> 31) == 0;
   const bool small = hi == 0;
-  const uint64_t h = small ? (uint64_t)low : (uint64_t)hi, rest = small ? 0ULL : (uint64_t)low << 32;
+  const uint64_t h = small ? (uint64_t)tail : (uint64_t)hi, rest = small ? 0ULL : (uint64_t)tail << 32;
   const int lead = __clzll((long long)h);  // 64 for zero
   const uint64_t top = (h << (lead & 63)) | ((rest >> 1) >> (63 - (lead & 63)));  // leading one at bit 63
   mant = (top >> 11) + ((top >> 10) & 1);                                         // 2^52 .. 2^53
-  e = (small ? 0 : 32) - lead + 11 + scale;                                       // value = mant 2^e
+  e = (small ? 0 : 32) - lead + 11 + top_field - 2112;                            // value = mant 2^e
   const int field = e + 1075;
   far = h != 0 && (field <= 0 || field >= 2046);
   const uint64_t bits = ((uint64_t)(uint32_t)(field - 1) << 52) + mant;
   return __longlong_as_double((long long)(h == 0 ? 0ULL : (bits | (uint64_t)neg << 63)));
+}
+
+// columns with an infinity or NaN (all lanes of a warp)
+__device__ __forceinline__ unsigned special_columns(const unsigned* s_col) {
+  return __ballot_sync(0xffffffffu, field_of(s_col[threadIdx.x & 31]) == 0x7ff);
+}
+
+// upper half of the magnitude of C's fixed-point number (k, n), to a unit: below 2^30, 2^26 is
+// an eighth of the power of two of the column's largest
+__device__ __forceinline__ unsigned upper_half(const uint64_t* Cf, int NT, int k, int n) {
+  const unsigned* const at = reinterpret_cast<const unsigned*>(Cf) + 1;
+  return (unsigned)abs((int)(at[2 * (((k >> 3) * NT + n) * 8 + (k & 7))] - 0x80808080u));
+}
+
+// The first n outputs of the queue (row << 5 | column), eight lanes each: whether two partners
+// are large enough for the digits, else the FP64 sum.  (These two stand out of line: inlined,
+// their registers cost the loop around them 10 %.)
+__device__ __noinline__ void settle(const double* __restrict__ in, const double* __restrict__ C, double* __restrict__ out,
+                                    int N, long long M, const unsigned* queue, int n, const uint64_t* Cf, int NT,
+                                    const unsigned* s_col) {
+  const int sub = threadIdx.x & 7;
+  const unsigned special = special_columns(s_col);
+  const unsigned mates = 0xffu << (threadIdx.x & 24);
+  for (int q = threadIdx.x >> 3; q < n; q += kTcThreads / 8) {
+    const unsigned w = queue[q];
+    const int c = (int)(w & 31u);
+    const double* __restrict__ a = in + (long long)(w >> 5) * N;
+    // the row's upper halves, their loads in flight together
+    int up[16];
+#pragma unroll
+    for (int x = 0; x < 16; ++x) up[x] = sub + 8 * x < N ? __ldg(reinterpret_cast<const int*>(a + sub + 8 * x) + 1) : 0;
+    int most = 0, er = 1;  // largest field less its partner's leading zeros, the row's largest field
+#pragma unroll
+    for (int x = 0; x < 16; ++x) {
+      if (sub + 8 * x >= N) break;
+      const int f = field_of(size_at(up[x], 0));
+      most = max(most, f > 0 ? f - __clz((int)upper_half(Cf, NT, 8 * x + sub, c)) : 0);
+      er = max(er, f);
+    }
+    for (int o = 1; o < 8; o <<= 1) {
+      most = max(most, __shfl_xor_sync(mates, most, o));
+      er = max(er, __shfl_xor_sync(mates, er, o));
+    }
+    if (!(special >> c & 1) && er < 0x7ff && most >= max(er - 5, 1)) continue;
+    double v = 0.0;
+    for (int k = sub; k < N; k += 8) v = fma(__ldg(a + k), __ldg(C + (long long)k * N + c), v);
+    for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(mates, v, o);
+    if (sub == 0) out[(long long)c * M + (w >> 5)] = v;
+  }
+}
+
+// A tile's `total` outputs marked in `weak`, summed in FP64, neighbours along a row.  All threads.
+__device__ __noinline__ void sum_many(const double* __restrict__ rows, const double* __restrict__ C, double* __restrict__ out,
+                                      int N, long long M, const unsigned* weak, int* before, int total) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int n[4], end = 0;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) end += n[x] = __popc(weak[4 * lane + x]);
+    int at = end;
+    for (int d = 1; d < 32; d <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, end, d);
+      if (lane >= d) end += t;
+    }
+    at = end - at;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      before[4 * lane + x] = at;
+      at += n[x];
+    }
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < total; q += kTcThreads) {
+    int lo = 0, hi = kTcRows - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) / 2;
+      if (before[mid] <= q) lo = mid;
+      else hi = mid - 1;
+    }
+    unsigned w = weak[lo];
+    for (int x = before[lo]; x < q; ++x) w &= w - 1;
+    const int c = __ffs((int)w) - 1;
+    const double* __restrict__ a = rows + (long long)lo * N;
+    double v = 0.0;
+    for (int k = 0; k < N; ++k) v = fma(__ldg(a + k), __ldg(C + (long long)k * N + c), v);
+    out[(long long)c * M + lo] = v;
+  }
 }
 
 // One quarter transform.  Block (x, y): the S tile y (its part of C stays in shared memory as
@@ -209,13 +311,18 @@ __device__ __forceinline__ double assemble(const uint32_t (*acc)[8], int col, in
 // the row tiles x, x + gridDim.x, ...  Per 16-wide k step the block stages the raw rows, cuts
 // them and C's share into digits and one thread issues the digit products; two blocks per SM
 // (256 of the 512 TMEM columns each) overlap one's products with the other's digits.
-// Bound by the integer work around the products: of a tile's ~34,000 cycles at N = 76 (two
-// blocks per SM) about 8,000 cut digits, 7,400 put results together, 7,500 find the row
-// exponents and 6,000 stage rows.  One product of N = 8 NT columns per row digit, instead of
-// one per digit pair, took issuing them from 2,400 to 150 cycles a step.  us per transform,
-// k_quarter -> this: N = 7 86 -> 34, 13 86 -> 41, 32 537 -> 81, 64 6,930 -> 1,020, 76
-// 28,980 -> 2,980, 100 91,700 -> 11,500, 128 219,500 -> 25,600 (FP64 arithmetic alone is
-// 16,000 at N = 76, memory 320).  C kept as digits: 76 2,915, 100 15,600, 128 38,000.
+// Bound by the integer work around the products: of a tile's ~41,000 cycles at N = 76 (two
+// blocks per SM) about 6,600 cut the rows' digits, 7,400 put results together, 7,500 find the
+// row exponents, 6,000 stage rows, 3,000 cut C's digits and make the products eight accumulators
+// wide, 4,000 look for weak outputs and 3,400 settle them (0.8 % of all).
+// One product of N = 8 NT columns per row digit, instead of one per digit pair, took issuing
+// them from 2,400 to 150 cycles a step.  us per transform of a dense tensor, k_quarter -> this
+// (without the look at weak outputs): N = 7 86 -> 47 (34), 13 86 -> 52 (41), 32 537 -> 100 (81),
+// 64 6,930 -> 1,240 (1,020), 76 28,980 -> 3,630 (2,980), 100 91,700 -> 14,200 (11,500), 128
+// 219,500 -> 30,700 (25,600); N = 76 with C in four blocks 7,040, C = 1 (everything weak but
+// the diagonal) 18,400.  FP64 arithmetic alone is 16,000 at N = 76, memory 320.  Weak outputs
+// settled tile by tile: 4,070 (one lane each), 4,550 (eight); one of the row's largest elements
+// looked at instead of two: 4,000.  C kept as digits: 76 -2 %, 100 +36 %, 128 +48 %.
 // Prefetching the next tile into L2 was slower up to N = 76.
 __global__ void __launch_bounds__(kTcThreads, 2)
     k_quarter_tc(const double* __restrict__ in, const double* __restrict__ C, double* __restrict__ out, int N,
@@ -223,8 +330,15 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ uint32_t s_tmem;
-  __shared__ int s_rows[2][kTcRows];  // largest exponent field of every row, this tile's and the next one's
-  __shared__ int s_col[kTcCols];
+  // largest size_at of every row, this tile's and the next one's, and the largest of the other
+  // half of its k; the largest of every column
+  __shared__ unsigned s_rows[2][kTcRows], s_other[2][kTcRows];
+  __shared__ unsigned s_col[kTcCols];
+  // outputs that the digits may not hold: this tile's columns of every row, how many before a row
+  // and in all (of two tiles in turn), and those kept until they fill the block (row << 5 | column)
+  __shared__ unsigned s_weak[kTcRows];
+  __shared__ int s_before[kTcRows], s_total[2], s_queued;
+  __shared__ unsigned s_queue[kTcQueue + kTcMany];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int steps = (N + 15) / 16, Kp = steps * 16;
   const int S0 = blockIdx.y * kTcCols, cols = min(kTcCols, N - S0), NT = (cols + 15) & ~15;
@@ -248,10 +362,13 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     unsigned top = 0;
     if (n < cols)
       for (int k = lane; k < N; k += 32)
-        top = max(top, (unsigned)__double2hiint(__ldg(C + (long long)k * N + S0 + n)) & 0x7fffffffu);
+        top = max(top, size_at(__double2hiint(__ldg(C + (long long)k * N + S0 + n)), k));
     top = __reduce_max_sync(0xffffffffu, top);
-    if (lane == 0) s_col[n] = max((int)(top >> 20), 1);
+    if (lane == 0) s_col[n] = at_least_one(top);
   }
+  if (tid < kTcRows) s_weak[tid] = 0u;
+  if (tid < 2) s_total[tid] = 0;
+  if (tid == 2) s_queued = 0;
   __syncthreads();
   const uint32_t tmem = s_tmem;
   for (int u = tid; u < NT * (Kp / 8); u += kTcThreads) {
@@ -259,7 +376,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int k = oct * 8 + j;
-      Cf[u * 8 + j] = fixed_digits(n < cols && k < N ? __ldg(C + (long long)k * N + S0 + n) : 0.0, s_col[n]);
+      Cf[u * 8 + j] = fixed_digits(n < cols && k < N ? __ldg(C + (long long)k * N + S0 + n) : 0.0, field_of(s_col[n]));
     }
   }
   for (int u = tid; u < 2 * (kTcDigits - 1) * NT; u += kTcThreads) {
@@ -270,9 +387,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   const uint32_t idesc = 1u << 4 | 1u << 7 | 1u << 10 | (uint32_t)(kTcDigits * NT >> 3) << 17 | (uint32_t)(kTcRows >> 4) << 24;
   uint32_t phase = 0;
   bool good = true;
-  // largest exponent of every row of the tile at m: a warp per 16 rows, their loads in flight
+  // largest size_at of every row of the tile at m: a warp per 16 rows, their loads in flight
   // together (row by row this took 25,000 of a tile's 54,000 cycles)
-  auto row_exponents = [&](long long m, int* to) {
+  auto row_exponents = [&](long long m, int to) {
     constexpr int R = kTcRows / 8;
     const int rows = (int)min((long long)kTcRows, M - m) - warp * R;
     const int* __restrict__ src = reinterpret_cast<const int*>(in + (m + warp * R) * N) + 1;  // high words
@@ -283,20 +400,24 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int* __restrict__ h = src + 2 * (r * N + k);
-        const unsigned u = r < rows ? (unsigned)__ldg(h) & 0x7fffffffu : 0u;
-        const unsigned w = r < rows && k + 32 < N ? (unsigned)__ldg(h + 64) & 0x7fffffffu : 0u;
+        const unsigned u = r < rows ? size_at(__ldg(h), k) : 0u;
+        const unsigned w = r < rows && k + 32 < N ? size_at(__ldg(h + 64), k + 32) : 0u;
         top[r] = max(top[r], max(u, w));
       }
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const unsigned v = __reduce_max_sync(0xffffffffu, top[r]);
-      if (lane == 0) to[warp * R + r] = max((int)(v >> 20), 1);
+      const unsigned even = __reduce_max_sync(0xffffffffu, lane & 1 ? 0u : top[r]);
+      const unsigned odd = __reduce_max_sync(0xffffffffu, lane & 1 ? top[r] : 0u);
+      if (lane == 0) {
+        s_rows[to][warp * R + r] = at_least_one(max(even, odd));
+        s_other[to][warp * R + r] = min(even, odd);
+      }
     }
   };
   const long long mstep = (long long)gridDim.x * kTcRows;
   int buf = 0;
-  if ((long long)blockIdx.x * kTcRows < M) row_exponents((long long)blockIdx.x * kTcRows, s_rows[0]);
+  if ((long long)blockIdx.x * kTcRows < M) row_exponents((long long)blockIdx.x * kTcRows, 0);
   const int lr = tid >> 4, lk = tid & 15;  // raw staging: row lr + 16 x, k lk
   const int row = tid & (kTcRows - 1), oct = tid >> 7;
   for (long long m0 = (long long)blockIdx.x * kTcRows; m0 < M; m0 += mstep, buf ^= 1) {
@@ -306,7 +427,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 #pragma unroll
     for (int x = 0; x < 8; ++x)
       nxt[x] = lr + 16 * x < rows && lk < N ? __ldg(src + (long long)(lr + 16 * x) * N + lk) : 0.0;
-    const int* const s_row = s_rows[buf];
+    const unsigned* const s_row = s_rows[buf];
     for (int st = 0; st < steps; ++st) {
 #pragma unroll
       for (int x = 0; x < 8; ++x) raw[(lr + 16 * x) * kTcRawStride + lk] = nxt[x];
@@ -325,7 +446,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         double x[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = raw[row * kTcRawStride + oct * 8 + j];
-        store_digits(x, s_row[row], As + (oct * kTcRows + row) * 16);
+        store_digits(x, field_of(s_row[row]), As + (oct * kTcRows + row) * 16);
         // C's digits of the step: a pair of k per thread
         for (int u = tid; u < 8 * NT; u += kTcThreads) {
           const ulonglong2 f = reinterpret_cast<const ulonglong2*>(Cf + (size_t)st * 16 * NT)[u];
@@ -338,6 +459,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncthreads();
       if (tid == 0) {
+        if (st == 0) s_total[buf ^ 1] = 0;  // (read before this tile's first barrier)
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         // the digits of C lie one after another along N, the accumulators one after another in
         // TMEM: digit i of the rows meets digits 0 .. 7 - i of C, added into accumulators i .. 7.
@@ -354,50 +476,91 @@ __global__ void __launch_bounds__(kTcThreads, 2)
                      : "memory");
       }
     }
-    if (m0 + mstep < M) row_exponents(m0 + mstep, s_rows[buf ^ 1]);  // beside the last products
+    if (m0 + mstep < M) row_exponents(m0 + mstep, buf ^ 1);  // beside the last products
     good = good && wait_phase(bar, phase);
     phase ^= 1;
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     // ---- outputs: lane = row of the warp's quarter, the two warps of a quarter share the columns
     const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * (NT / 2);
-    const int er = s_row[r];
+    const unsigned big = s_row[r], big2 = s_other[buf][r];
+    const int er = field_of(big);
+    const unsigned special = special_columns(s_col);
+    const int widest = __reduce_max_sync(0xffffffffu, field_of(s_col[lane])), gap = er - field_of(big2);
+    const unsigned need = big >= 1u << 20 ? 1u << 26 : ~0u, need2 = big2 >= 1u << 20 && gap <= 3 ? 1u << (26 + gap) : ~0u;
+    unsigned mine = 0;
     for (int c = c0; c < c0 + NT / 2; c += 8) {
       uint32_t acc[kTcDigits][8];
 #pragma unroll
       for (int d = 0; d < kTcDigits; ++d)
         tmem_load8(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(d * NT + c), acc[d]);
       double v[8];
-      unsigned odd = 0;  // columns that the common path does not cover
+      unsigned out_of = 0, weak = 0;  // columns outside the normal doubles; the digits may not hold them
 #pragma unroll
       for (int x = 0; x < 8; ++x) {
-        const int ec = s_col[c + x];
-        bool far, neg;
+        bool far, low, neg;
         uint64_t mant;
         int e;
-        v[x] = assemble(acc, x, er + ec - 2168 + 56, far, neg, mant, e);
-        odd |= (far || er == 0x7ff || ec == 0x7ff ? 1u : 0u) << x;
+        v[x] = assemble(acc, x, er + field_of(s_col[c + x]), far, low, neg, mant, e);
+        out_of |= (far ? 1u : 0u) << x;
+        weak |= (low ? 1u : 0u) << x;
       }
-      if (odd) {
+      const int left = cols - c;
+      const unsigned real = r < rows && left > 0 ? (left >= 8 ? 0xffu : (1u << left) - 1u) : 0u;
+      // (all er + ec up to 1027: what is left out is below half a unit of the subnormals per k)
+      weak &= er + widest <= 1027 ? 0u : real;
+      // one of the row's two largest elements meets a partner that makes the product large enough:
+      // nine in ten end here
+      out_of &= real;
+      for (unsigned todo = weak; todo; todo &= todo - 1) {
+        const int x = __ffs((int)todo) - 1;
+        if (upper_half(Cf, NT, big & 127, c + x) >= need || upper_half(Cf, NT, big2 & 127, c + x) >= need2) weak &= ~(1u << x);
+      }
+      weak |= er == 0x7ff ? real : special >> c & real;
+      if (out_of) {
 #pragma unroll
         for (int x = 0; x < 8; ++x) {
-          const int ec = s_col[c + x];
-          if (!(odd >> x & 1) || c + x >= cols || r >= rows) continue;
-          bool far, neg;
+          if (!(out_of >> x & 1)) continue;
+          bool far, low, neg;
           uint64_t mant;
           int e;
-          assemble(acc, x, er + ec - 2168 + 56, far, neg, mant, e);
-          if (er == 0x7ff || ec == 0x7ff) v[x] = plain_dot(src + (long long)r * N, C + S0 + c + x, N);
-          else v[x] = neg ? -scaled(mant, e) : scaled(mant, e);
+          assemble(acc, x, er + field_of(s_col[c + x]), far, low, neg, mant, e);
+          v[x] = neg ? -scaled(mant, e) : scaled(mant, e);
         }
       }
+      reinterpret_cast<unsigned char*>(s_weak + r)[c >> 3] = (unsigned char)weak;
+      mine |= weak << (c - c0);
 #pragma unroll
       for (int x = 0; x < 8; ++x)
-        if (c + x < cols && r < rows)
+        if (real >> x & 1)
           out[(long long)(S0 + c + x) * M + m0 + r] = good ? v[x] : __longlong_as_double(0x7ff8000000000000LL);
     }
+    const int some = __reduce_add_sync(0xffffffffu, __popc(mine)), queued = s_queued;
+    if (lane == 0 && some) atomicAdd(&s_total[buf], some);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();  // accumulators, exponents and raw rows are free again
+    const int total = s_total[buf];
+    if (total == 0) continue;
+    // ---- the weak outputs: a few wait for those of the next tiles, as many as fill the block
+    // (eight warps waiting for one cost 40 % at N = 76); many are summed at once, without a look at
+    // their partners, neighbours along a row
+    if (total <= kTcMany) {
+      if (queued >= kTcQueue) {
+        settle(in, C + S0, out + (long long)S0 * M, N, M, s_queue, queued, Cf, NT, s_col);
+        __syncthreads();
+        if (tid == 0) s_queued = 0;
+        __syncthreads();
+      }
+      if (mine) {
+        int at = atomicAdd(&s_queued, __popc(mine));
+        for (unsigned todo = mine; todo; todo &= todo - 1)
+          s_queue[at++] = (unsigned)(m0 + r) << 5 | (unsigned)(c0 + __ffs((int)todo) - 1);
+      }
+      continue;
+    }
+    sum_many(src, C + S0, out + (long long)S0 * M + m0, N, M, s_weak, s_before, total);
   }
+  __syncthreads();
+  settle(in, C + S0, out + (long long)S0 * M, N, M, s_queue, s_queued, Cf, NT, s_col);
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTcTmem));
 }
