@@ -1447,16 +1447,18 @@ extern "C" int mmdg_set_screen(mmdg_context* h, const double* screen, long long 
 //     reads each P_sr once for all of them;
 //   K blocks take one p and a run of rows q, their (q, r) positions flattened over the
 //     threads (kKPos each, so N need not be a multiple of 32), one accumulator per position
-//     over the loop over s; the positions of a row are added up at the end.
+//     over the loop over s; the positions of a row are added up at the end (above N = 512 a block
+//     takes its one row in parts).
 // One warp per (p, q) with lanes over (r, s), the exchange at a stride of N^2 elements, took
 // 749 us at N = 100 (42 at N = 50), this form 369 (34).  Measured beside it: 4 or 16 rows
 // per J block 379 / 370, 4 positions per thread 375 and 48 at N = 50.
-constexpr int kJKThreads = 256, kJRows = 8, kKPos = 2;
+constexpr int kJKThreads = 256, kJRows = 8, kKPos = 2, kJKPositions = kJKThreads * kKPos;
 
+template <bool LONG>  // N > 512 (the loop over parts costs 5 % at N = 100)
 __global__ void __launch_bounds__(kJKThreads) k_jk_dense(const double* __restrict__ T, const double* __restrict__ P,
                                                          double* __restrict__ J, double* __restrict__ K, int N, int nj,
                                                          int qrows, int qblocks) {
-  __shared__ double sum[kJKThreads * kKPos];
+  __shared__ double sum[kJKPositions];
   const long long NN = (long long)N * N;
   if ((int)blockIdx.x < nj) {
     const long long row0 = (long long)blockIdx.x * kJRows;
@@ -1505,32 +1507,41 @@ __global__ void __launch_bounds__(kJKThreads) k_jk_dense(const double* __restric
   const int b = (int)blockIdx.x - nj, p = b / qblocks, q0 = (b - p * qblocks) * qrows;
   const int nq = min(qrows, N - q0), npos = nq * N;
   const double* __restrict__ t = T + (long long)p * NN * N + (long long)q0 * N;  // + s N^2 + position
-  double acc[kKPos];
-  int r[kKPos];
-#pragma unroll
-  for (int x = 0; x < kKPos; ++x) {
-    acc[x] = 0.0;
-    r[x] = (int)(threadIdx.x + x * kJKThreads) % N;
-  }
-#pragma unroll 4
-  for (int s = 0; s < N; ++s) {
-    const double* __restrict__ ts = t + s * NN;
-    const double* __restrict__ ps = P + (long long)s * N;
+  const int lane = threadIdx.x & 31;
+  double rest = 0.0;  // of a row longer than a block's positions: its earlier ones, in the first warp
+  for (int at = 0; at < (LONG ? npos : 1); at += kJKPositions) {
+    double acc[kKPos];
+    int r[kKPos];
 #pragma unroll
     for (int x = 0; x < kKPos; ++x) {
-      const int pos = threadIdx.x + x * kJKThreads;
-      if (pos < npos) acc[x] = fma(__ldcs(ts + pos), __ldg(ps + r[x]), acc[x]);
+      acc[x] = 0.0;
+      r[x] = (int)(at + threadIdx.x + x * kJKThreads) % N;
     }
-  }
+#pragma unroll 4
+    for (int s = 0; s < N; ++s) {
+      const double* __restrict__ ts = t + s * NN;
+      const double* __restrict__ ps = P + (long long)s * N;
 #pragma unroll
-  for (int x = 0; x < kKPos; ++x) sum[threadIdx.x + x * kJKThreads] = acc[x];
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  for (int q = threadIdx.x >> 5; q < nq; q += kJKThreads / 32) {
-    double v = 0.0;
-    for (int x = lane; x < N; x += 32) v += sum[q * N + x];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) K[(long long)p * N + q0 + q] = v;
+      for (int x = 0; x < kKPos; ++x) {
+        const int pos = at + threadIdx.x + x * kJKThreads;
+        if (pos < npos) acc[x] = fma(__ldcs(ts + pos), __ldg(ps + r[x]), acc[x]);
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < kKPos; ++x) sum[threadIdx.x + x * kJKThreads] = acc[x];
+    __syncthreads();
+    const int end = min(N, npos - at);  // positions of a row here: N, or what is left of the one row
+    for (int q = threadIdx.x >> 5; q < nq; q += kJKThreads / 32) {
+      double v = LONG ? rest : 0.0;
+      for (int x = lane; x < (LONG ? min(end, kJKPositions) : N); x += 32) v += sum[q * N + x];
+      if (LONG && at + kJKPositions < npos) {
+        rest = v;
+        continue;
+      }
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) K[(long long)p * N + q0 + q] = v;
+    }
+    if (LONG) __syncthreads();
   }
 }
 
@@ -1538,11 +1549,10 @@ extern "C" int mmdg_jk_dense(mmdg_context* h, long long N, const double* T, cons
                              void* stream) {
   if (!h || !T || !P || !J || !K || N <= 0) return fail(MMDG_E_ARG, "mmdg_jk_dense: bad argument");
   DeviceGuard dg(h->device);
-  // (a K block holds at least one row: N^4 elements of a larger N are past any memory)
-  if (N > kJKThreads * kKPos) return fail(MMDG_E_ARG, "mmdg_jk_dense: N above 512");
   const int n = (int)N, nj = (int)((N * N + kJRows - 1) / kJRows);
-  const int qrows = std::min(n, kJKThreads * kKPos / n), qblocks = (n + qrows - 1) / qrows;
-  k_jk_dense<<<nj + n * qblocks, kJKThreads, 0, (cudaStream_t)stream>>>(T, P, J, K, n, nj, qrows, qblocks);
+  const int qrows = std::max(1, std::min(n, kJKPositions / n)), qblocks = (n + qrows - 1) / qrows;
+  const auto kernel = n > kJKPositions ? k_jk_dense<true> : k_jk_dense<false>;
+  kernel<<<nj + n * qblocks, kJKThreads, 0, (cudaStream_t)stream>>>(T, P, J, K, n, nj, qrows, qblocks);
   CUDA_TRY(cudaGetLastError());
   return MMDG_OK;
 }
