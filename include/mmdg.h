@@ -253,12 +253,15 @@ int mmdg_mlp_adam_many(int count, float* const* w, void* const* w_bf16, const fl
 /* AO -> MO transform of an ERI tensor (mmd/postscf.py:26-27, four einsums with the MO
  * coefficients): eri_out[P,Q,R,S] = sum_pqrs C[p,P] C[q,Q] C[r,R] C[s,S] eri_in[p,q,r,s].
  * All device arrays, C order: C is N x N (AO row, MO column), eri_in / eri_out / work
- * are N^4 and distinct; eri_in is left unchanged, work is scratch.  Four FP64 quarter
- * transforms (each contracts the last index and writes the new one first). */
+ * are N^4 and distinct; eri_in is left unchanged, work is scratch.  Four quarter
+ * transforms (each contracts the last index and writes the new one first), above N = 128
+ * by FP64 FMAs, up to it from digit products on the tensor cores with FP64 sums where
+ * those hold too few digits: in both forms an element of a quarter transform (a normal
+ * double) is within N 2^-53 sum_s |in_s| |C_s| of the exact sum, then rounded. */
 int mmdg_ao2mo(long long N, const double* C, const double* eri_in, double* eri_out, double* work, void* stream);
 
 /* The ERI kernels' reciprocal square root (an FP32 estimate refined by one
- * third-order FP64 step) and CUDA's rsqrt at n points, for x in the normal float
+ * third-order step) and CUDA's rsqrt at n points, for x in the normal float
  * range (device arrays).  Test support; no counterpart in the reference. */
 int mmdg_rsqrt(mmdg_context* ctx, long long n, const double* x, double* ours, double* cuda, void* stream);
 

@@ -557,8 +557,9 @@ static std::vector<int> group_counts(const std::vector<int>& vals, const std::ve
 }
 
 // lanes per pair (as a power of two) of the Schwarz kernel, whose heaviest pair has `most`
-// primitive pairs: a lane keeps about four of its most^2 primitive quartets.  One thread
-// per pair was a serial chain of up to 1296 of them, 1.35 ms of (H2O)8's set-up.
+// primitive pairs: enough that a lane keeps four of its most^2 primitive quartets at the most, up
+// to a warp (then 40 of 1296).  One thread per pair was a serial chain of all 1296, 1.35 ms of
+// (H2O)8's set-up.
 static int schwarz_lanes(int most) {
   int lg = 0;
   while (lg < 5 && (long long)most * most > (4LL << lg)) ++lg;
@@ -1274,9 +1275,11 @@ static int fock_impl(mmdg_context* h, const double* dP, double* G, double tol, d
     CUDA_TRY(cudaEventRecord(h->fork_ev, st));
     for (int k = 0; k < ns; ++k) CUDA_TRY(cudaStreamWaitEvent(h->side[k], h->fork_ev, 0));
   }
-  // small molecules: highest angular momentum first, whose few quartets are the longest chains
-  // ((H2O)4 6-31G** 1.21 -> 1.16 ms); large ones: the long lists first ((H2O)16 39.6, reversed
-  // 39.9; mixed 19.1, 19.4).  The line lies between 0.7 and 171 million candidates.
+  // small molecules: highest angular momentum first, whose few quartets are the longest chains;
+  // large ones: the long lists first.  ms per build of n waters 6-31G**, chains first / long lists
+  // first: 2 0.51 / 0.54, 4 (0.7 million candidates) 1.06 / 1.11, 5 1.68 / 1.71, 6 (3.5 million)
+  // 2.96 / 2.95, 7 (6.5 million) 4.63 / 4.60, 8 6.29 / 6.24, 12 17.9 / 17.8, 16 39.9 / 39.6;
+  // increments with FP32 below 1e-5: 4 1.05 / 1.22, 6 2.08 / 2.15, 8 3.65 / 3.66, 10 5.65 / 5.58.
   const bool chains_first = !class_ms && h->q_total < (4 << 20);
   for (int k = 0; k < MMDG_NCLASS; ++k) {
     const int ci = chains_first ? MMDG_NCLASS - 1 - k : k;

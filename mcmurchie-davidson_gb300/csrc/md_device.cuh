@@ -54,24 +54,6 @@ __device__ __forceinline__ double f64_of_positive(float y) {
   return __hiloint2double((((b >> 23) + (1023 - 127)) << 20) | ((b & 0x7fffff) >> 3), (b & 7) << 29);
 }
 
-// a finite float as a double, exactly, on the integer pipe (zero and subnormal: 0)
-__device__ __forceinline__ double f64_of_float(float x) {
-  const int b = __float_as_int(x);
-  const int e = (b >> 23) & 0xff;
-  if (e == 0) return 0.0;
-  return __hiloint2double((b & 0x80000000) | ((e + (1023 - 127)) << 20) | ((b & 0x7fffff) >> 3), (b & 7) << 29);
-}
-
-// a double as a float rounded toward zero, sign kept, on the integer pipe (relative
-// error below 2^-23; magnitudes below the normal float range give 0)
-__device__ __forceinline__ float f32_of_double_tz(double x) {
-  const int hi = __double2hiint(x);
-  const unsigned lo = (unsigned)__double2loint(x);
-  const int fe = min(((hi >> 20) & 0x7ff) - (1023 - 127), 254);
-  return fe <= 0 ? 0.0f
-                 : __int_as_float((hi & 0x80000000) | (fe << 23) | ((hi & 0xfffff) << 3) | (int)(lo >> 29));
-}
-
 // an unevaluated sum of two floats (see the double-float arithmetic below)
 struct DF {
   float hi, lo;

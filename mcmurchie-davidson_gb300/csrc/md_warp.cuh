@@ -141,9 +141,9 @@ __global__ void __launch_bounds__(kThreads) k_fock_warp(Geometry g, FockArgs f, 
   const unsigned nwarps = gridDim.x * kWarps;
   const unsigned cap = max_item > 0 ? (unsigned)max_item : (unsigned)kItem;  // autotuned, or kItem
   const int item = (int)max(1u, min(cap, n / (4u * nwarps)));
-  // (claimed one at a time: claiming the next item ahead, as k_fock does, was slower
-  // here -- (dp|pp) 2.55 against 3.2 ms per (H2O)16 build -- since a warp then holds
-  // two items of up to 8 quartets each when the list runs out)
+  // (claimed one at a time: claiming the next item ahead was slower -- (dp|pp) 2.55 against
+  // 3.2 ms per (H2O)16 build -- since a warp then holds two items of up to 8 quartets each when
+  // the list runs out)
   for (;;) {
     unsigned long long claim = 0;
     if (lane == 0) claim = atomicAdd(f.work, (unsigned long long)item);

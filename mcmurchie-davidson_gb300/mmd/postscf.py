@@ -2,8 +2,9 @@
 ``mmd.postscf.PostSCF`` API (mmd/postscf.py:13-73).
 
 ``PostSCF(mol)`` requires a converged conventional RHF (the device ERI tensor) and
-runs ``ao2mo``: the 4-index transform (pq|rs) -> (PQ|RS) as four FP64 quarter
-transforms over one index each (the project's kernel, mmdg_ao2mo), the
+runs ``ao2mo``: the 4-index transform (pq|rs) -> (PQ|RS) as four quarter
+transforms over one index each (the project's kernel, mmdg_ao2mo: double precision, up to
+N = 128 from exact digit products on the tensor cores), the
 spin-orbital antisymmetrised integrals <AB||CD> (spin orbital 2p + sigma, the
 ordering of the reference's Kronecker products; built on first use), the spin-orbital
 core Hamiltonian ``Hp`` and orbital energies ``fs`` -- the attributes the reference
